@@ -73,6 +73,9 @@ struct st_chain {
   size_t zsmem = 0;
   double* d_injected = nullptr;
   size_t injected_n = 0;
+  bool count = false;      // the sweep's Z pass is the counting pass (st_zcount.cuh)
+  bool ct_tuned = false;   // its tile came from the autotuner or from st_model
+  long ct_cap = 0;         // CTAs its scratch has room for
   int tile_min_t = 0;      // Z-pass tiles the scratch was sized for: T >= tile_min_t,
   int tile_min_r = 1;      // R >= tile_min_r (fast path; the autotuner stays inside)
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -86,8 +89,9 @@ struct st_chain {
 struct ZGroup {
   int first = 0, n = 0;    // slice of the batch table
   int KT = 0, W = 8;
-  size_t zsmem = 0;
-  int tz = 0;              // CTAs of the slice
+  bool count = false;      // counting pass (zsmem_ct, tzc, pzc) or the general one only
+  size_t zsmem = 0, zsmem_ct = 0;
+  int tz = 0, tzc = 0;     // CTAs of the slice: general pass, counting pass
   bool same = false;       // one data set and tile for the whole slice (kZfInterleave)
 };
 
@@ -96,6 +100,7 @@ struct st_batch {
   std::vector<st_chain*> chains;   // sorted by K class
   ChainDev* d_table = nullptr;
   int* d_pz = nullptr;     // prefix: Z pass (restarting at 0 in every group)
+  int* d_pzc = nullptr;    // prefix: counting Z pass (likewise)
   int* d_pl = nullptr;     // prefix: locus kernel (over d_table_l)
   ChainDev* d_table_l = nullptr;   // the table in the locus kernel's CTA order
   int* d_pi = nullptr;     // prefix: individual kernel
@@ -109,7 +114,7 @@ struct st_batch {
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   std::vector<ChainDev> table;             // host copies of the device tables
   std::vector<ChainDev> table_l;
-  std::vector<int> pz, pl, pi;
+  std::vector<int> pz, pzc, pl, pi;
   std::vector<cudaStream_t> aux;           // one per K class (several classes only)
   cudaEvent_t ev_fork = nullptr;
   std::vector<cudaEvent_t> ev_join;
@@ -308,12 +313,24 @@ void choose_tile(const st_model* m, int N, int L, int K, int* T, int* W, int* R)
   *R = r;
 }
 
+void set_count_tile(ChainDev* h, CountTile t) {
+  h->ct_like_magic = zcount_like_magic(h->N, h->L);
+  h->ctT = t.T;
+  h->ctR = t.R;
+  h->ctchunks = (h->N + t.T - 1) / t.T;
+  h->ctgroups = (int)(zcount_ctas(h->N, h->L, t) / h->ctchunks);
+}
+
 int zpass(st_chain* c, int mode, int flags) {
   Bracket br(c->ctx, mode == kZMetro ? ST_K_METRO : (mode == kZNormal ? ST_K_ZPASS : ST_K_OTHER));
   st_ctx* ctx = c->ctx;
   if (mode == kZNormal || mode == kZInit || mode == kZRecount) {
     ST_CUDA(ctx, cudaMemsetAsync(c->h.npart, 0, sizeof(int32_t) * (size_t)c->h.K * c->h.A * c->h.L, ctx->stream));
     ST_CUDA(ctx, cudaMemsetAsync(c->h.mpart, 0, sizeof(int32_t) * (size_t)c->h.N * c->h.K, ctx->stream));
+  }
+  if (c->count && mode == kZNormal) {
+    LaunchSet ls = single(c, c->h.ctchunks * c->h.ctgroups);
+    return cuda_check(c->ctx, launch_zcount(ls, c->KT, flags, zcount_smem(c->KT, c->h.ctT)), "zcount");
   }
   if (c->fast) {
     LaunchSet ls = single(c, ctas_zpass_b2g(c->h));
@@ -376,13 +393,16 @@ int check_model(st_ctx* ctx, const st_model* m) {
 
 }  // namespace
 
-// The Z-pass tile a chain of this shape gets by default (st_model tile fields
-// zero), for callers without a chain (st_update_z_noalloc).
-void st::default_zpass_tile(int N, int L, int K, int* T, int* W, int* R) {
+// CTAs of the general Z pass at the tile a chain of this shape gets by default
+// (st_model tile fields zero), for callers without a chain (st_update_z_noalloc).
+long st::default_zpass_ctas(int N, int L, int K) {
   st_model m{};
   st_model_defaults(&m);
   m.tile_t = m.tile_w = m.tile_r = 0;
-  choose_tile(&m, N, L, K, T, W, R);
+  int T, W, R;
+  choose_tile(&m, N, L, K, &T, &W, &R);
+  const long lblocks = (L + 32 * W - 1) / (32 * W);
+  return (N + T - 1) / T * ((lblocks + R - 1) / R);
 }
 
 // ===========================================================================
@@ -855,6 +875,8 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
     const int lblocks = (L + 32 * W - 1) / (32 * W);
     h.ngroups = (lblocks + R - 1) / R;
     c->zsmem = zpass_smem_all(c->KT, K, T, W);
+    c->count = !model->store_z && !model->pfrompopflagonly;
+    c->ct_tuned = model->tile_t > 0 || model->tile_r > 0;
   } else {
     h.tileT = N; h.tileW = 8; h.tileR = 1;
     h.nchunks = 1;
@@ -877,10 +899,17 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
   ChainDev hw = h;
   hw.G = 32;  // scratch sized for the widest group a batch may impose
   const int nred = std::max(ctas_locus(hw, kBlockLoc) * K, ctas_ind(hw, kBlockInd) * (K + 1));
+  if (c->count) {
+    // per-CTA partials of the Z pass and of the update kernels share one region
+    c->ct_cap = (long)zctas + nred;
+    const CountTile t = zcount_tile(N, L, c->KT, model->tile_t, model->tile_r, 1, c->ct_cap);
+    if (t.T > 0) set_count_tile(&h, t);
+    else c->count = false;
+  }
   struct Buf { void** p; size_t bytes; };
   void *Q, *logQ, *TQ, *lTQ, *P, *logP, *eps, *F, *alpha, *lambda, *Z = nullptr, *npart, *mpart,
       *ldpart, *QSum, *PSum, *SumEps, *FstSum, *sumAlpha, *sumlambda, *AD = nullptr, *stats,
-      *likepart, *redpart, *ctr, *rep, *err, *chain, *prefix;
+      *partials, *ctr, *rep, *err, *chain, *prefix;
   std::vector<Buf> bufs = {
       {&Q, NK * 4}, {&logQ, NK * 4}, {&TQ, NK * 4}, {&lTQ, NK * 4}, {&P, LKA * 4},
       {&logP, LKA * 4}, {&eps, LA * 8}, {&F, (size_t)K * 8}, {&alpha, arows * K * 8},
@@ -888,7 +917,7 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
       {&mpart, NK * 4}, {&ldpart, (size_t)h.ngroups * N * 8},
       {&QSum, NK * 8}, {&PSum, LKA * 8}, {&SumEps, LA * 8}, {&FstSum, (size_t)K * 8},
       {&sumAlpha, arows * K * 8}, {&sumlambda, (size_t)K * 8}, {&stats, (size_t)kStSize * 8},
-      {&likepart, (size_t)zctas * 8}, {&redpart, (size_t)nred * 8},
+      {&partials, ((size_t)zctas + nred) * 8},
       {&ctr, (size_t)kCtrCount * 4}, {&rep, 4}, {&err, 4}, {&chain, sizeof(ChainDev)},
       {&prefix, 16}};
   if (model->store_z) bufs.push_back({&Z, (size_t)N * 2 * L});
@@ -960,8 +989,8 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
   h.npart = (int32_t*)npart; h.mpart = (int32_t*)mpart; h.ldpart = (double*)ldpart;
   h.QSum = (double*)QSum; h.PSum = (double*)PSum; h.SumEps = (double*)SumEps;
   h.FstSum = (double*)FstSum; h.sumAlpha = (double*)sumAlpha; h.sumlambda = (double*)sumlambda;
-  h.AncestDist = (int32_t*)AD; h.stats = (double*)stats; h.likepart = (double*)likepart;
-  h.redpart = (double*)redpart; h.ctr = (unsigned*)ctr; h.rep = (int*)rep; h.err = (int*)err;
+  h.AncestDist = (int32_t*)AD; h.stats = (double*)stats; h.likepart = (double*)partials;
+  h.redpart = (double*)partials; h.ctr = (unsigned*)ctr; h.rep = (int*)rep; h.err = (int*)err;
   c->d_chain = (ChainDev*)chain;
   c->d_prefix = (int*)prefix;
   data->chains++;
@@ -1475,7 +1504,9 @@ extern "C" int st_get_state(st_chain* c, int f, void* host, size_t bytes) {
   const ChainDev& h = c->h;
   if (f == ST_F_REP) { memcpy(host, &c->host_rep, 4); return ST_OK; }
   if (f == ST_F_DIMS) {
-    int32_t d[8] = {h.N, h.L, h.K, h.A, h.layout, h.G, h.nchunks, h.ngroups};
+    // the tile of the sweep's Z pass
+    int32_t d[8] = {h.N, h.L, h.K, h.A, h.layout, h.G, c->count ? h.ctchunks : h.nchunks,
+                    c->count ? h.ctgroups : h.ngroups};
     memcpy(host, d, 32);
     return ST_OK;
   }
@@ -1585,20 +1616,23 @@ static int batch_layout(st_batch* b, bool keep_groups) {
   const int n = (int)b->chains.size();
   b->table.assign(n, ChainDev{});
   b->pz.assign(n, 0);
+  b->pzc.assign(n, 0);
   b->pl.assign(n, 0);
   b->pi.assign(n, 0);
   b->tz = b->tl = b->ti = 0;
   if (!keep_groups) b->zg.clear();
-  for (ZGroup& g : b->zg) { g.tz = 0; g.zsmem = 0; g.n = 0; }
+  for (ZGroup& g : b->zg) { g.tz = g.tzc = 0; g.zsmem = g.zsmem_ct = 0; g.n = 0; }
   size_t gi = 0;
   for (int j = 0; j < n; j++) {
     st_chain* c = b->chains[j];
     b->table[j] = c->h;
     b->table[j].G = b->G;   // every chain's kernels index their groups by the batch-wide G
     if (b->fast) {
-      if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT)) {
+      if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT ||
+                           b->zg.back().count != c->count)) {
         ZGroup g;
         g.first = j;
+        g.count = c->count;
         g.KT = c->KT;
         g.W = c->h.tileW;
         b->zg.push_back(g);
@@ -1610,6 +1644,14 @@ static int batch_layout(st_batch* b, bool keep_groups) {
       b->pz[j] = g.tz;
       g.tz += ctas_zpass_b2g(b->table[j]);
       g.zsmem = std::max(g.zsmem, c->zsmem);
+      if (g.count) {
+        // a tile for the batch's CTAs together, unless one was tuned or given
+        if (!c->ct_tuned)
+          set_count_tile(&b->table[j], zcount_tile(c->h.N, c->h.L, c->KT, 0, 0, n, c->ct_cap));
+        b->pzc[j] = g.tzc;
+        g.tzc += b->table[j].ctchunks * b->table[j].ctgroups;
+        g.zsmem_ct = std::max(g.zsmem_ct, zcount_smem(c->KT, b->table[j].ctT));
+      }
       g.n++;
     } else {
       b->pz[j] = b->tz;
@@ -1625,7 +1667,7 @@ static int batch_layout(st_batch* b, bool keep_groups) {
       const ChainDev& h = b->table[j];
       g.same = g.same && h.g2 == h0.g2 && h.N == h0.N && h.L == h0.L && h.wpr == h0.wpr &&
                h.tileT == h0.tileT && h.tileR == h0.tileR && h.nchunks == h0.nchunks &&
-               h.ngroups == h0.ngroups;
+               h.ngroups == h0.ngroups && h.ctT == h0.ctT && h.ctR == h0.ctR;
     }
   }
   // locus kernel: chains whose CTAs take longest first (longest-processing-
@@ -1658,6 +1700,7 @@ static void batch_upload(st_batch* b) {
   const int n = (int)b->chains.size();
   cudaMemcpy(b->d_table, b->table.data(), sizeof(ChainDev) * n, cudaMemcpyHostToDevice);
   cudaMemcpy(b->d_pz, b->pz.data(), 4 * n, cudaMemcpyHostToDevice);
+  cudaMemcpy(b->d_pzc, b->pzc.data(), 4 * n, cudaMemcpyHostToDevice);
   cudaMemcpy(b->d_pl, b->pl.data(), 4 * n, cudaMemcpyHostToDevice);
   cudaMemcpy(b->d_table_l, b->table_l.data(), sizeof(ChainDev) * n, cudaMemcpyHostToDevice);
   cudaMemcpy(b->d_pi, b->pi.data(), 4 * n, cudaMemcpyHostToDevice);
@@ -1680,6 +1723,20 @@ static bool set_tile(st_chain* c, int T, int R) {
 }
 
 static bool apply_group_tile(st_batch* b, const ZGroup& g, int T, int R) {
+  if (g.count) {
+    std::vector<CountTile> t;
+    for (int j = g.first; j < g.first + g.n; j++) {
+      const st_chain* c = b->chains[j];
+      t.push_back(zcount_tile(c->h.N, c->h.L, g.KT, T, R, 1, c->ct_cap));
+      if (t.back().T <= 0) return false;
+    }
+    for (int j = g.first; j < g.first + g.n; j++) {
+      set_count_tile(&b->chains[j]->h, t[j - g.first]);
+      b->chains[j]->ct_tuned = true;
+      upload_chain(b->chains[j]);
+    }
+    return true;
+  }
   for (int j = g.first; j < g.first + g.n; j++) {
     st_chain* c = b->chains[j];
     const int t0 = c->h.tileT, r0 = c->h.tileR;
@@ -1697,16 +1754,18 @@ static bool apply_group_tile(st_batch* b, const ZGroup& g, int T, int R) {
 // group's chains.
 struct TileKey {
   int KT;
+  bool count;   // tile of the counting pass (R unused) or of the general one
   std::vector<int64_t> shapes;
   bool operator<(const TileKey& o) const {
-    return KT != o.KT ? KT < o.KT : shapes < o.shapes;
+    if (KT != o.KT) return KT < o.KT;
+    return count != o.count ? count < o.count : shapes < o.shapes;
   }
 };
 static std::mutex g_tile_mu;
 static std::map<TileKey, std::pair<int, int>> g_tile_cache;
 
 static TileKey tile_key(st_batch* b, const ZGroup& g) {
-  TileKey k{g.KT, {}};
+  TileKey k{g.KT, g.count, {}};
   for (int j = g.first; j < g.first + g.n; j++)
     k.shapes.push_back(((int64_t)b->chains[j]->h.N << 32) | (uint32_t)b->chains[j]->h.L);
   return k;
@@ -1734,7 +1793,9 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
   b->chains.assign(chains, chains + n);
   // one Z launch per K class: keep each class contiguous in the table
   std::stable_sort(b->chains.begin(), b->chains.end(),
-                   [](const st_chain* a, const st_chain* c) { return a->KT < c->KT; });
+                   [](const st_chain* a, const st_chain* c) {
+                     return a->KT != c->KT ? a->KT < c->KT : a->count < c->count;
+                   });
   st_chain* c0 = b->chains[0];
   b->fast = c0->fast;
   int G = 1;
@@ -1762,6 +1823,7 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
     return e == cudaSuccess ? ST_OK : seterr(ctx, ST_ERR_NOMEM, "batch table");
   };
   if (alloc((void**)&b->d_table, sizeof(ChainDev) * n) || alloc((void**)&b->d_pz, 4 * n) ||
+      alloc((void**)&b->d_pzc, 4 * n) ||
       alloc((void**)&b->d_pl, 4 * n) || alloc((void**)&b->d_pi, 4 * n) ||
       alloc((void**)&b->d_table_l, sizeof(ChainDev) * n)) {
     st_batch_destroy(b);
@@ -1839,10 +1901,12 @@ extern "C" int st_batch_autotune(st_batch* b, int reps) {
   for (size_t gi = 0; gi < b->zg.size() && rc == ST_OK; gi++) {
     ZGroup& g = b->zg[gi];
     st_chain* c0 = b->chains[g.first];
-    const int T0 = c0->h.tileT, R0 = c0->h.tileR;
+    const int T0 = g.count ? b->table[g.first].ctT : c0->h.tileT;
+    const int R0 = g.count ? b->table[g.first].ctR : c0->h.tileR;
     std::vector<std::pair<int, int>> cand;
     for (int tm : {2, 3, 4, 5, 6, 8})
       for (int rm : {1, 2, 4, 8}) {
+        if (g.count && rm > 1) continue;   // one locus block per CTA
         const std::pair<int, int> tr{((T0 * tm / 4) + 15) & ~15, R0 * rm};
         if (std::find(cand.begin(), cand.end(), tr) == cand.end()) cand.push_back(tr);
       }
@@ -1852,7 +1916,8 @@ extern "C" int st_batch_autotune(st_batch* b, int reps) {
       if (!apply_group_tile(b, g, tr.first, tr.second)) continue;
       batch_layout(b, true);
       batch_upload(b);
-      LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, s};
+      LaunchSet lg{b->d_table + g.first, (g.count ? b->d_pzc : b->d_pz) + g.first, g.n,
+                   g.count ? g.tzc : g.tz, s};
       double ms_sum = 0.0;
       for (int r = 0; r <= reps && rc == ST_OK; r++) {
         for (int j = g.first; j < g.first + g.n; j++) {
@@ -1861,8 +1926,9 @@ extern "C" int st_batch_autotune(st_batch* b, int reps) {
           cudaMemsetAsync(h.mpart, 0, (size_t)h.N * h.K * 4, s);
         }
         cudaEventRecord(e0, s);
-        cudaError_t e = launch_zpass_b2g(lg, g.KT, g.W, kZNormal, g.same ? kZfInterleave : 0,
-                                         g.zsmem);
+        const int fl = g.same ? kZfInterleave : 0;
+        cudaError_t e = g.count ? launch_zcount(lg, g.KT, fl, g.zsmem_ct)
+                                : launch_zpass_b2g(lg, g.KT, g.W, kZNormal, fl, g.zsmem);
         cudaEventRecord(e1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         if (e != cudaSuccess) rc = cuda_check(ctx, e, "autotune");
@@ -1898,7 +1964,7 @@ extern "C" int st_batch_autotune(st_batch* b, int reps) {
 extern "C" int st_batch_destroy(st_batch* b) {
   if (!b) return ST_ERR_ARG;
   cudaSetDevice(b->ctx->device);
-  for (void* p : {(void*)b->d_table, (void*)b->d_pz, (void*)b->d_pl, (void*)b->d_pi,
+  for (void* p : {(void*)b->d_table, (void*)b->d_pz, (void*)b->d_pzc, (void*)b->d_pl, (void*)b->d_pi,
                   (void*)b->d_table_l})
     if (p) cudaFree(p);
   if (b->ev0) cudaEventDestroy(b->ev0);
@@ -1933,9 +1999,14 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
       const ZGroup& g = b->zg[gi];
       cudaStream_t gs = fork ? b->aux[gi] : s;
       if (fork) ST_CUDA(ctx, cudaStreamWaitEvent(gs, b->ev_fork, 0));
-      LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, gs};
-      ST_CUDA(ctx, launch_zpass_b2g(lg, g.KT, g.W, mode, flags | (g.same ? kZfInterleave : 0),
-                                    g.zsmem));
+      const int fl = flags | (g.same ? kZfInterleave : 0);
+      if (g.count && mode == kZNormal) {
+        LaunchSet lg{b->d_table + g.first, b->d_pzc + g.first, g.n, g.tzc, gs};
+        ST_CUDA(ctx, launch_zcount(lg, g.KT, fl, g.zsmem_ct));
+      } else {
+        LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, gs};
+        ST_CUDA(ctx, launch_zpass_b2g(lg, g.KT, g.W, mode, fl, g.zsmem));
+      }
       if (fork) ST_CUDA(ctx, cudaEventRecord(b->ev_join[gi], gs));
     }
     if (fork)

@@ -49,6 +49,7 @@ __device__ __forceinline__ U4 philox_s(uint32_t a, uint32_t b, uint32_t rep,
 struct PhiloxRun {
   uint32_t head;         // hi(M1 rep) ^ k0_0 ^ (stream << 24)
   uint32_t y1, z0, z2, w3;
+  __device__ __forceinline__ PhiloxRun() {}
   __device__ __forceinline__ PhiloxRun(uint32_t a, uint32_t rep, uint32_t stream,
                                        uint32_t seed32) {
     const uint64_t p0 = (uint64_t)0xD2511F53u * a, p1 = (uint64_t)0xCD9E8D57u * rep;
@@ -63,6 +64,22 @@ struct PhiloxRun {
     z2 = (uint32_t)(q2 >> 32) ^ (kPhiloxKey1 + 2u * 0xBB67AE85u);
     w3 = (uint32_t)q2 ^ (kPhiloxKey1 + 3u * 0xBB67AE85u);
   }
+  // a ^ b ^ KEY as one three-input operation with the key as its immediate: left
+  // to itself the code generator keeps the key schedule in registers and steps
+  // it with two additions per round.
+  template <uint32_t KEY>
+  static __device__ __forceinline__ uint32_t xor_key(uint32_t a, uint32_t b) {
+    uint32_t d;
+    asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(d) : "r"(a), "r"(b), "n"(KEY));
+    return d;
+  }
+  template <int R>
+  static __device__ __forceinline__ void rounds_from(U4& c) {
+    const uint64_t q0 = (uint64_t)0xD2511F53u * c.x, q1 = (uint64_t)0xCD9E8D57u * c.z;
+    c = U4{xor_key<kPhiloxKey0 + (uint32_t)R * 0x9E3779B9u>((uint32_t)(q1 >> 32), c.y), (uint32_t)q1,
+           xor_key<kPhiloxKey1 + (uint32_t)R * 0xBB67AE85u>((uint32_t)(q0 >> 32), c.w), (uint32_t)q0};
+    if constexpr (R < 9) rounds_from<R + 1>(c);
+  }
   __device__ __forceinline__ U4 block_r0(uint32_t c0) const {
     const uint64_t r1 = (uint64_t)0xD2511F53u * c0;                     // round 1
     const uint32_t r1c2 = (uint32_t)(r1 >> 32) ^ y1, r1c3 = (uint32_t)r1;
@@ -70,19 +87,10 @@ struct PhiloxRun {
     const uint32_t r2c0 = (uint32_t)(r2 >> 32) ^ z0, r2c1 = (uint32_t)r2, r2c2 = r1c3 ^ z2;
     const uint64_t p0 = (uint64_t)0xD2511F53u * r2c0;                   // round 3
     const uint64_t p1 = (uint64_t)0xCD9E8D57u * r2c2;
-    uint32_t c0n = (uint32_t)(p1 >> 32) ^ r2c1 ^ (kPhiloxKey0 + 3u * 0x9E3779B9u);
-    uint32_t c1n = (uint32_t)p1, c2n = (uint32_t)(p0 >> 32) ^ w3, c3n = (uint32_t)p0;
-#pragma unroll
-    for (int r = 4; r < 10; r++) {
-      const uint32_t k0 = kPhiloxKey0 + (uint32_t)r * 0x9E3779B9u;
-      const uint32_t k1 = kPhiloxKey1 + (uint32_t)r * 0xBB67AE85u;
-      const uint64_t q0 = (uint64_t)0xD2511F53u * c0n;
-      const uint64_t q1 = (uint64_t)0xCD9E8D57u * c2n;
-      const uint32_t n0 = (uint32_t)(q1 >> 32) ^ c1n ^ k0;
-      const uint32_t n2 = (uint32_t)(q0 >> 32) ^ c3n ^ k1;
-      c0n = n0; c1n = (uint32_t)q1; c2n = n2; c3n = (uint32_t)q0;
-    }
-    return U4{c0n, c1n, c2n, c3n};
+    U4 c{xor_key<kPhiloxKey0 + 3u * 0x9E3779B9u>((uint32_t)(p1 >> 32), r2c1), (uint32_t)p1,
+         (uint32_t)(p0 >> 32) ^ w3, (uint32_t)p0};
+    rounds_from<4>(c);
+    return c;
   }
   __device__ __forceinline__ U4 block(uint32_t b) const { return block_r0(head ^ (b & 0xFFFFFFu)); }
 };

@@ -39,12 +39,26 @@ enum : int { kIndGibbs = 0, kIndPropose = 1, kIndAccept = 2, kIndNone = 3 };
 enum : int { kIndAlpha = 0x1, kIndCollect = 0x2 };
 
 size_t zpass_b2g_smem(int KT, int K, int T, int W, int mode);
-// The default Z-pass tile (T individuals, W warps, R locus blocks) of a chain
-// of this shape (st_api.cu choose_tile).
-void default_zpass_tile(int N, int L, int K, int* T, int* W, int* R);
+// CTAs of the general Z pass at its default tile for a chain of this shape
+// (st_api.cu choose_tile).
+long default_zpass_ctas(int N, int L, int K);
 int zpass_b2g_width(int KT);   // CTA width (warps) of the fast path for a K class
 cudaError_t launch_zpass_b2g(const LaunchSet& ls, int KT, int W, int mode, int flags,
                              size_t smem);
+// The sweep's counting Z pass (biallelic data, no stored Z, every individual's
+// alleles counted).  A tile is T individuals x R blocks of 256 loci per CTA.
+struct CountTile { int T, R; };
+constexpr int kZcountMinT = 32, kZcountMaxT = 512;
+constexpr int kZcountMaxR = 127;   // 16-bit row counts: 512 copies per block
+size_t zcount_smem(int KT, int T);
+bool zcount_fits(int KT, int T);
+long zcount_ctas(int N, int L, CountTile t);
+// The tile for `chains` chains of this shape in one launch, with at most `cap` CTAs a
+// chain (room for their ln P(D) partials); tile_t, tile_r: the caller's choice, or 0.
+// T = 0: no tile fits.
+CountTile zcount_tile(int N, int L, int KT, int tile_t, int tile_r, int chains, long cap);
+double zcount_like_magic(int N, int L);
+cudaError_t launch_zcount(const LaunchSet& ls, int KT, int flags, size_t smem);
 cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags);
 cudaError_t launch_locus(const LaunchSet& ls, int stages, int block);
 cudaError_t launch_ind(const LaunchSet& ls, int G, int mode, int stages, int block);

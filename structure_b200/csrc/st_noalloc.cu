@@ -106,23 +106,23 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
         const float* P, uint64_t seed, int rep, int32_t* n_out, int32_t* m_out,
         double* like_out, int32_t* err_out, cudaStream_t stream, size_t* scratch_bytes) {
   const int KT = k_class(K);
-  int T, W, R;
-  default_zpass_tile(N, L, K, &T, &W, &R);   // the tile a chain of this shape gets
-  const int nchunks = (N + T - 1) / T;
-  const int lblocks = (L + 32 * W - 1) / (32 * W);
-  const int ngroups = (lblocks + R - 1) / R;
-  const size_t ntiles = (size_t)nchunks * ngroups;
-
-  // scratch layout: head | stats | likepart | n histogram | m histogram
-  const size_t o_stats = align256(sizeof(Head));
-  const size_t o_like = o_stats + align256(sizeof(double) * kStSize);
-  const size_t o_n = o_like + align256(sizeof(double) * ntiles);
+  // scratch layout: head | stats | n histogram | m histogram | ln P(D) partials.
+  // A problem is admitted by what the general Z pass' partials would take, and the
+  // counting pass gets a tile whose partials fit what is there.
   const size_t nbytes = sizeof(int32_t) * (size_t)K * 2 * L;
   const size_t mbytes = sizeof(int32_t) * (size_t)N * K;
+  const size_t o_stats = align256(sizeof(Head));
+  const size_t o_n = o_stats + align256(sizeof(double) * kStSize);
   const size_t o_m = o_n + align256(nbytes);
-  const size_t need = o_m + align256(mbytes);
+  const size_t o_like = o_m + align256(mbytes);
+  const size_t need = o_like + align256(sizeof(double) * (size_t)default_zpass_ctas(N, L, K));
   if (scratch_bytes) *scratch_bytes = need;
   if (need > kScratchBytes) return ST_ERR_ADMISSION;
+  const CountTile t =
+      zcount_tile(N, L, KT, 0, 0, 1, (long)((kScratchBytes - o_like) / sizeof(double)));
+  if (t.T <= 0) return ST_ERR_ADMISSION;
+  const int nchunks = (N + t.T - 1) / t.T;
+  const long ntiles = zcount_ctas(N, L, t);
 
   void* base = nullptr;
   int rc = scratch_addr(device, &base);
@@ -146,8 +146,8 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
     z ^= z >> 31;
     h.key = (uint32_t)z;
   }
-  h.tileT = T; h.tileW = W; h.tileR = R;
-  h.nchunks = nchunks; h.ngroups = ngroups;
+  h.ct_like_magic = zcount_like_magic(N, L);
+  h.ctT = t.T; h.ctR = t.R; h.ctchunks = nchunks; h.ctgroups = (int)(ntiles / nchunks);
   h.cnt_chunks = 1; h.cnt_groups = 1;
   h.g2 = g2;
   h.Q = const_cast<float*>(Q);
@@ -176,8 +176,7 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
   ls.nchains = 1;
   ls.total_ctas = (int)ntiles;
   ls.stream = stream;
-  const size_t smem = zpass_b2g_smem(KT, K, T, W, kZNormal);
-  if (launch_zpass_b2g(ls, KT, W, kZNormal, like_out ? kZfLikeAlways : 0, smem) != cudaSuccess)
+  if (launch_zcount(ls, KT, like_out ? kZfLikeAlways : 0, zcount_smem(KT, t.T)) != cudaSuccess)
     return ST_ERR_CUDA;
 
   const size_t total = (size_t)K * 2 * L + (size_t)N * K;

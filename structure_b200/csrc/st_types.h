@@ -71,6 +71,10 @@ struct ChainDev {
   // count histogram slices summed by the consumers (1: every producer adds
   // into slice 0); Metropolis log-ratio partials have ngroups slices
   int cnt_chunks, cnt_groups;
+  // tile of the counting Z pass: individuals per chunk, locus blocks per CTA, and
+  // the chunks and locus groups they make
+  int ctT, ctR, ctchunks, ctgroups;
+  double ct_like_magic;     // rounds a word's ln P(D) to the chain's quantum (zcount_like_magic)
   // data
   const uint32_t* g2;
   const uint8_t* g8;
@@ -89,7 +93,7 @@ struct ChainDev {
   double *QSum, *PSum, *SumEps, *FstSum, *sumAlpha, *sumlambda;
   int32_t* AncestDist;                  // N*K*numboxes
   double* stats;                        // kStSize
-  double *likepart, *redpart;           // per-CTA partials
+  double *likepart, *redpart;           // per-CTA partials (one region: used in turn)
   unsigned* ctr;                        // kCtrCount
   int* rep;                             // device sweep counter
   int* err;                             // device error word

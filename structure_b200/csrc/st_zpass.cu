@@ -17,6 +17,7 @@
 //   n[k][a][l] and m[i][k], with integer reductions (cleared by the host
 //   before the pass); the Metropolis log ratios leave as per-CTA partials
 //   ldpart[group][i].
+#include <cmath>
 #include <cstdio>
 #include "st_device.cuh"
 #include "st_kernels.h"
@@ -85,6 +86,93 @@ cudaError_t launch_zpass_b2g(const LaunchSet& ls, int KT, int W, int mode, int f
     ST_KCASE(1, 8) ST_KCASE(2, 8) ST_KCASE(3, 8) ST_KCASE(4, 8) ST_KCASE(5, 8) ST_KCASE(6, 8)
     ST_KCASE(7, 8) ST_KCASE(8, 8) ST_KCASE(9, 8) ST_KCASE(10, 8) ST_KCASE(11, 8) ST_KCASE(12, 8)
     ST_KCASE(16, 2) ST_KCASE(20, 2) ST_KCASE(24, 2) ST_KCASE(32, 2)
+#undef ST_KCASE
+  }
+  return cudaErrorInvalidValue;
+}
+
+namespace zcount {
+template <int KT>
+cudaError_t launch_zcount_k(const LaunchSet& ls, int flags, size_t smem);
+size_t zc_layout_total(int kt, int T);
+int zc_ctas_of(int kt);
+}  // namespace zcount
+
+size_t zcount_smem(int KT, int T) { return zcount::zc_layout_total(KT, T); }
+bool zcount_fits(int KT, int T) {
+  return T >= kZcountMinT && T <= kZcountMaxT && T % 16 == 0 && zcount_smem(KT, T) <= 200 * 1024;
+}
+long zcount_ctas(int N, int L, CountTile t) {
+  const long blocks = (L + 255) / 256;   // 8 warps of 32 loci
+  return (blocks + t.R - 1) / t.R * ((N + t.T - 1) / t.T);
+}
+
+// Individuals per chunk: the count of equal chunks with the least estimated time.  A
+// CTA costs its rows plus about 24 rows of fixed work per locus block (measured at
+// K=5: 128 rows 4 % above 256, 336 rows 1 % below); CTAs that share an SM share its
+// pipes, with fewer of them using it less fully (K=5: 2 instead of 3 CTAs 12 %
+// slower, 1 about 35 %).  A grid within one wave takes as long as its fullest SM; a
+// longer one, its mean plus half a wave of tail.  Several locus blocks per CTA save
+// next to nothing (0.3 % at K=5): R only keeps the CTAs within their partials.
+CountTile zcount_tile(int N, int L, int KT, int tile_t, int tile_r, int chains, long cap) {
+  const int np = (N + 15) & ~15;
+  auto with_r = [&](int T) {
+    CountTile t{T, tile_r > 0 ? (tile_r < kZcountMaxR ? tile_r : kZcountMaxR) : 1};
+    while (t.R < kZcountMaxR && zcount_ctas(N, L, t) > cap) t.R++;
+    return t;
+  };
+  CountTile best{0, 1};
+  if (tile_t > 0) {
+    int T = (tile_t + 15) & ~15;
+    T = T > np ? np : T;
+    T = T > kZcountMaxT ? kZcountMaxT : T < kZcountMinT ? kZcountMinT : T;
+    while (T > kZcountMinT && !zcount_fits(KT, T)) T -= 16;
+    const CountTile t = with_r(T);
+    return zcount_ctas(N, L, t) <= cap ? t : best;
+  }
+  double best_t = 1e300;
+  for (int n = 1; n <= (np + kZcountMinT - 1) / kZcountMinT; n++) {
+    int T = ((N + n - 1) / n + 15) & ~15;
+    if (T < kZcountMinT) T = kZcountMinT;
+    if (!zcount_fits(KT, T)) continue;
+    const CountTile c = with_r(T);
+    const long ctas1 = zcount_ctas(N, L, c);
+    if (ctas1 > cap) continue;
+    int occ = (int)((227 * 1024) / (zcount_smem(KT, T) + 1024 + 64));
+    if (occ > zcount::zc_ctas_of(KT)) occ = zcount::zc_ctas_of(KT);
+    const long ctas = ctas1 * chains, per_sm = (ctas + 147) / 148;
+    const int live = per_sm < occ ? (int)per_sm : occ;
+    const double eff = live >= 3 ? 1.0 : live == 2 ? 1.12 : 1.35;
+    const double n_sm = per_sm <= occ ? (double)per_sm : (double)ctas / 148.0 + 0.5 * occ;
+    const double t = n_sm * eff * c.R * (T + 24);
+    if (t < best_t) {
+      best_t = t;
+      best = c;
+    }
+    if (T <= kZcountMinT) break;
+  }
+  return best;
+}
+
+// ln P(D) is the sum of one FP32 value per genotype word (16 genotypes of a locus).
+// Rounded to a common quantum 2^-(47 - log2 words), the values add exactly in FP64
+// while they average below 32, so the sum does not depend on the tile: a batch and a
+// chain alone, at their own tiles, get the same bits.  The quantum is far below the
+// words' own FP32 rounding (2^-24 at 2^23 words of about 10 +- 2^-21).  Adding and
+// subtracting 1.5 x 2^52 quanta rounds to it.
+double zcount_like_magic(int N, int L) {
+  const double words = (double)L * ((N + 15) / 16);
+  int lg = 0;
+  while (lg < 46 && (double)(1ull << lg) < words) lg++;
+  return ldexp(1.5, 52 - (47 - lg));
+}
+
+cudaError_t launch_zcount(const LaunchSet& ls, int KT, int flags, size_t smem) {
+  switch (KT) {
+#define ST_KCASE(k) case k: return zcount::launch_zcount_k<k>(ls, flags, smem);
+    ST_KCASE(1) ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(5) ST_KCASE(6) ST_KCASE(7) ST_KCASE(8)
+    ST_KCASE(9) ST_KCASE(10) ST_KCASE(11) ST_KCASE(12) ST_KCASE(16) ST_KCASE(20) ST_KCASE(24)
+    ST_KCASE(32)
 #undef ST_KCASE
   }
   return cudaErrorInvalidValue;

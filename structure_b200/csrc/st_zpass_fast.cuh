@@ -604,8 +604,12 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
       ZArgs za{&ch, grow, Xlane, sQ2, sT2, sLD + warp * nT16, sInc, sM, mycol, i0, i1, nT16, l,
                K, L, lane,
                my_word, my_shift, prep, key, stream, valid, pfonly, store_z};
-      const bool ext = store_z || pfonly;
-      if (want_like) {
+      [[maybe_unused]] const bool ext = store_z || pfonly;
+      if constexpr (MODE == kZNormal) {
+        // chains with neither feature take the counting pass of st_zcount.cuh
+        if (want_like) zword_loop<KT, MODE, W, true, true>(za, like_acc, errb, p0r, p1r);
+        else zword_loop<KT, MODE, W, false, true>(za, like_acc, errb, p0r, p1r);
+      } else if (want_like) {
         if (ext) zword_loop<KT, MODE, W, true, true>(za, like_acc, errb, p0r, p1r);
         else zword_loop<KT, MODE, W, true, false>(za, like_acc, errb, p0r, p1r);
       } else {
