@@ -15,7 +15,7 @@ ROOT = os.path.dirname(HERE)
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libstgpu.so")
-SOURCES = ["st_zpass.cu", "st_zpass_k1.cu", "st_zpass_k2.cu", "st_zpass_k3.cu",
+SOURCES = ["st_zpass.cu", "st_zpass_u8.cu", "st_zpass_k1.cu", "st_zpass_k2.cu", "st_zpass_k3.cu",
            "st_zpass_k4.cu", "st_zpass_k5.cu", "st_zpass_k6.cu", "st_zcount_k1.cu", "st_zcount_k2.cu",
            "st_zcount_k3.cu", "st_zcount_k4.cu", "st_zcount_k5.cu", "st_zcount_k6.cu",
            "st_zcount_k7.cu", "st_update.cu", "st_api.cu",

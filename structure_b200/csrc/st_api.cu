@@ -74,6 +74,7 @@ struct st_chain {
   double* d_injected = nullptr;
   size_t injected_n = 0;
   bool count = false;      // the sweep's Z pass is the counting pass (st_zcount.cuh)
+  bool u8 = false;         // one-byte layout with FP32 draws (st_zpass_u8.cu), class KT
   bool ct_tuned = false;   // its tile came from the autotuner or from st_model
   long ct_cap = 0;         // CTAs its scratch has room for
   int tile_min_t = 0;      // Z-pass tiles the scratch was sized for: T >= tile_min_t,
@@ -108,6 +109,7 @@ struct st_batch {
   std::vector<ZGroup> zg;  // fast path: one Z launch per K class
   int G = 1;
   bool fast = false;
+  bool u8 = false;         // every chain takes st_zpass_u8.cu (one Z launch per K class)
   bool graphs = true;                          // replay captured sweeps
   cudaGraphExec_t gx[2] = {nullptr, nullptr};  // [Gibbs sweep, Metropolis sweep]
   int glaunches[2] = {0, 0};
@@ -321,6 +323,8 @@ void set_count_tile(ChainDev* h, CountTile t) {
   h->ctgroups = (int)(zcount_ctas(h->N, h->L, t) / h->ctchunks);
 }
 
+bool u8_mode(int mode) { return mode == kZNormal || mode == kZLike || mode == kZMetro; }
+
 int zpass(st_chain* c, int mode, int flags) {
   Bracket br(c->ctx, mode == kZMetro ? ST_K_METRO : (mode == kZNormal ? ST_K_ZPASS : ST_K_OTHER));
   st_ctx* ctx = c->ctx;
@@ -339,6 +343,10 @@ int zpass(st_chain* c, int mode, int flags) {
   }
   if (mode == kZMetro)
     ST_CUDA(ctx, cudaMemsetAsync(c->h.ldpart, 0, sizeof(double) * (size_t)c->h.N, ctx->stream));
+  if (c->u8 && u8_mode(mode) && !(flags & (kZfF64 | kZfInjected))) {
+    LaunchSet ls = single(c, ctas_u8(c->h));
+    return cuda_check(ctx, launch_u8(ls, c->KT, mode, flags, u8_smem(c->h, mode)), "zpass_u8");
+  }
   if (c->model.precision == 1) flags |= kZfF64;
   LaunchSet ls = single(c, ctas_zpass_u8(c->h, 256));
   return cuda_check(ctx, launch_zpass_u8(ls, mode, flags), "zpass_u8");
@@ -905,6 +913,14 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
     const CountTile t = zcount_tile(N, L, c->KT, model->tile_t, model->tile_r, 1, c->ct_cap);
     if (t.T > 0) set_count_tile(&h, t);
     else c->count = false;
+  }
+  if (!c->fast && model->precision == 0) {
+    h.u8_lc = u8_plan(N, L, K, A, (long)zctas + nred);
+    c->u8 = h.u8_lc > 0;
+    if (c->u8) {
+      h.u8_chunks = (L + h.u8_lc - 1) / h.u8_lc;
+      c->KT = u8_kclass(K);
+    }
   }
   struct Buf { void** p; size_t bytes; };
   void *Q, *logQ, *TQ, *lTQ, *P, *logP, *eps, *F, *alpha, *lambda, *Z = nullptr, *npart, *mpart,
@@ -1627,7 +1643,20 @@ static int batch_layout(st_batch* b, bool keep_groups) {
     st_chain* c = b->chains[j];
     b->table[j] = c->h;
     b->table[j].G = b->G;   // every chain's kernels index their groups by the batch-wide G
-    if (b->fast) {
+    if (!b->fast && b->u8) {
+      if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT)) {
+        ZGroup g;
+        g.first = j;
+        g.KT = c->KT;
+        b->zg.push_back(g);
+      }
+      ZGroup& g = b->zg.back();   // (the autotuner, which keeps groups, has no tiles here)
+      b->pz[j] = g.tz;
+      g.tz += ctas_u8(b->table[j]);
+      g.zsmem = std::max(g.zsmem, u8_smem(c->h, kZNormal));
+      g.zsmem_ct = std::max(g.zsmem_ct, u8_smem(c->h, kZMetro));
+      g.n++;
+    } else if (b->fast) {
       if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT ||
                            b->zg.back().count != c->count)) {
         ZGroup g;
@@ -1798,6 +1827,8 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
                    });
   st_chain* c0 = b->chains[0];
   b->fast = c0->fast;
+  b->u8 = !c0->fast;
+  for (st_chain* c : b->chains) b->u8 = b->u8 && c->u8;
   int G = 1;
   for (st_chain* c : b->chains) {
     if (c->ctx != ctx || c->fast != b->fast || c->h.metrofreq != c0->h.metrofreq ||
@@ -1841,7 +1872,7 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
   batch_upload(b);
   cudaEventCreate(&b->ev0);
   cudaEventCreate(&b->ev1);
-  if (b->fast && b->zg.size() > 1) {
+  if (b->zg.size() > 1) {
     cudaEventCreateWithFlags(&b->ev_fork, cudaEventDisableTiming);
     for (size_t gi = 0; gi < b->zg.size(); gi++) {
       cudaStream_t as = nullptr;
@@ -1989,10 +2020,9 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
   st_chain* c0 = b->chains[0];
   cudaStream_t s = ctx->stream;
   LaunchSet lz{b->d_table, b->d_pz, n, b->tz, s};
-  // one fast Z launch per K class over its slice of the table
-  // one fast Z launch per K class; with several classes they run side by side
+  // one Z launch per K class over its slice of the table; with several classes they run side by side
   // on forked streams (independent chains), so one class's tail overlaps the next
-  auto zfast = [&](int mode, int flags) -> int {
+  auto zgroups = [&](int mode, int flags) -> int {
     const bool fork = b->zg.size() > 1 && !b->aux.empty();
     if (fork) ST_CUDA(ctx, cudaEventRecord(b->ev_fork, s));
     for (size_t gi = 0; gi < b->zg.size(); gi++) {
@@ -2000,7 +2030,10 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
       cudaStream_t gs = fork ? b->aux[gi] : s;
       if (fork) ST_CUDA(ctx, cudaStreamWaitEvent(gs, b->ev_fork, 0));
       const int fl = flags | (g.same ? kZfInterleave : 0);
-      if (g.count && mode == kZNormal) {
+      if (b->u8) {
+        LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, gs};
+        ST_CUDA(ctx, launch_u8(lg, g.KT, mode, flags, mode == kZMetro ? g.zsmem_ct : g.zsmem));
+      } else if (g.count && mode == kZNormal) {
         LaunchSet lg{b->d_table + g.first, b->d_pzc + g.first, g.n, g.tzc, gs};
         ST_CUDA(ctx, launch_zcount(lg, g.KT, fl, g.zsmem_ct));
       } else {
@@ -2045,8 +2078,8 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
         ST_CUDA(ctx, cudaMemsetAsync(c->h.ldpart, 0, sizeof(double) * c->h.N, s));
     {
       Bracket br(ctx, ST_K_METRO);
-      if (b->fast) {
-        if (int rc = zfast(kZMetro, 0)) return rc;
+      if (b->fast || b->u8) {
+        if (int rc = zgroups(kZMetro, 0)) return rc;
       } else {
         ST_CUDA(ctx, launch_zpass_u8(lz, kZMetro, c0->model.precision ? kZfF64 : 0));
       }
@@ -2085,8 +2118,8 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
   }
   {
     Bracket br(ctx, ST_K_ZPASS);
-    if (b->fast) {
-      if (int rc = zfast(kZNormal, zflags)) return rc;
+    if (b->fast || b->u8) {
+      if (int rc = zgroups(kZNormal, zflags)) return rc;
     } else {
       ST_CUDA(ctx, launch_zpass_u8(lz, kZNormal, zflags | (c0->model.precision ? kZfF64 : 0)));
     }

@@ -21,18 +21,30 @@ struct U4 { uint32_t x, y, z, w; };
 
 constexpr uint32_t kPhiloxKey0 = 0xA511E9B3u, kPhiloxKey1 = 0x3C6EF372u;
 
+// a ^ b ^ KEY as one three-input operation with the key as its immediate: left to
+// itself the code generator keeps the key schedule in registers and steps it with
+// two additions per round (a tenth of the Z pass' instructions).
+template <uint32_t KEY>
+__device__ __forceinline__ uint32_t xor_key(uint32_t a, uint32_t b) {
+  uint32_t d;
+  asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(d) : "r"(a), "r"(b), "n"(KEY));
+  return d;
+}
+
+// Philox rounds R..9.
+template <int R>
+__device__ __forceinline__ void philox_rounds(U4& c) {
+  const uint64_t p0 = (uint64_t)0xD2511F53u * c.x;   // one 32x32->64 multiply each
+  const uint64_t p1 = (uint64_t)0xCD9E8D57u * c.z;
+  c = U4{xor_key<kPhiloxKey0 + (uint32_t)R * 0x9E3779B9u>((uint32_t)(p1 >> 32), c.y), (uint32_t)p1,
+         xor_key<kPhiloxKey1 + (uint32_t)R * 0xBB67AE85u>((uint32_t)(p0 >> 32), c.w), (uint32_t)p0};
+  if constexpr (R < 9) philox_rounds<R + 1>(c);
+}
+
 __device__ __forceinline__ U4 philox(uint32_t c0, uint32_t c1, uint32_t c2, uint32_t c3) {
-#pragma unroll
-  for (int r = 0; r < 10; r++) {
-    const uint32_t k0 = kPhiloxKey0 + (uint32_t)r * 0x9E3779B9u;
-    const uint32_t k1 = kPhiloxKey1 + (uint32_t)r * 0xBB67AE85u;
-    const uint64_t p0 = (uint64_t)0xD2511F53u * c0;   // one 32x32->64 multiply each
-    const uint64_t p1 = (uint64_t)0xCD9E8D57u * c2;
-    const uint32_t n0 = (uint32_t)(p1 >> 32) ^ c1 ^ k0;
-    const uint32_t n2 = (uint32_t)(p0 >> 32) ^ c3 ^ k1;
-    c0 = n0; c1 = (uint32_t)p1; c2 = n2; c3 = (uint32_t)p0;
-  }
-  return U4{c0, c1, c2, c3};
+  U4 c{c0, c1, c2, c3};
+  philox_rounds<0>(c);
+  return c;
 }
 
 __device__ __forceinline__ U4 philox_s(uint32_t a, uint32_t b, uint32_t rep,
@@ -64,22 +76,6 @@ struct PhiloxRun {
     z2 = (uint32_t)(q2 >> 32) ^ (kPhiloxKey1 + 2u * 0xBB67AE85u);
     w3 = (uint32_t)q2 ^ (kPhiloxKey1 + 3u * 0xBB67AE85u);
   }
-  // a ^ b ^ KEY as one three-input operation with the key as its immediate: left
-  // to itself the code generator keeps the key schedule in registers and steps
-  // it with two additions per round.
-  template <uint32_t KEY>
-  static __device__ __forceinline__ uint32_t xor_key(uint32_t a, uint32_t b) {
-    uint32_t d;
-    asm("lop3.b32 %0, %1, %2, %3, 0x96;" : "=r"(d) : "r"(a), "r"(b), "n"(KEY));
-    return d;
-  }
-  template <int R>
-  static __device__ __forceinline__ void rounds_from(U4& c) {
-    const uint64_t q0 = (uint64_t)0xD2511F53u * c.x, q1 = (uint64_t)0xCD9E8D57u * c.z;
-    c = U4{xor_key<kPhiloxKey0 + (uint32_t)R * 0x9E3779B9u>((uint32_t)(q1 >> 32), c.y), (uint32_t)q1,
-           xor_key<kPhiloxKey1 + (uint32_t)R * 0xBB67AE85u>((uint32_t)(q0 >> 32), c.w), (uint32_t)q0};
-    if constexpr (R < 9) rounds_from<R + 1>(c);
-  }
   __device__ __forceinline__ U4 block_r0(uint32_t c0) const {
     const uint64_t r1 = (uint64_t)0xD2511F53u * c0;                     // round 1
     const uint32_t r1c2 = (uint32_t)(r1 >> 32) ^ y1, r1c3 = (uint32_t)r1;
@@ -89,7 +85,7 @@ struct PhiloxRun {
     const uint64_t p1 = (uint64_t)0xCD9E8D57u * r2c2;
     U4 c{xor_key<kPhiloxKey0 + 3u * 0x9E3779B9u>((uint32_t)(p1 >> 32), r2c1), (uint32_t)p1,
          (uint32_t)(p0 >> 32) ^ w3, (uint32_t)p0};
-    rounds_from<4>(c);
+    philox_rounds<4>(c);
     return c;
   }
   __device__ __forceinline__ U4 block(uint32_t b) const { return block_r0(head ^ (b & 0xFFFFFFu)); }

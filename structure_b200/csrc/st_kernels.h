@@ -60,6 +60,13 @@ CountTile zcount_tile(int N, int L, int KT, int tile_t, int tile_r, int chains, 
 double zcount_like_magic(int N, int L);
 cudaError_t launch_zcount(const LaunchSet& ls, int KT, int flags, size_t smem);
 cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags);
+// One-byte layout, FP32 draws (st_zpass_u8.cu): modes kZNormal, kZLike and kZMetro.
+// u8_plan chooses the loci per chunk with at most `cap` CTAs; 0 if it cannot.
+int u8_plan(int N, int L, int K, int A, long cap);
+int ctas_u8(const ChainDev& c);
+size_t u8_smem(const ChainDev& c, int mode);
+cudaError_t launch_u8(const LaunchSet& ls, int KT, int mode, int flags, size_t smem);
+int u8_kclass(int K);
 cudaError_t launch_locus(const LaunchSet& ls, int stages, int block);
 cudaError_t launch_ind(const LaunchSet& ls, int G, int mode, int stages, int block);
 cudaError_t launch_collect(const LaunchSet& ls, int block);

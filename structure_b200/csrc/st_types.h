@@ -68,6 +68,7 @@ struct ChainDev {
   int loc_tpl;              // locus kernel: lanes per locus (power of two, 1..32)
   // Z-pass tiling: T individuals per chunk, W warps, R locus blocks per CTA
   int tileT, tileW, tileR, nchunks, ngroups;
+  int u8_lc, u8_chunks;     // one-byte layout's Z pass: loci per chunk, chunks
   // count histogram slices summed by the consumers (1: every producer adds
   // into slice 0); Metropolis log-ratio partials have ngroups slices
   int cnt_chunks, cnt_groups;

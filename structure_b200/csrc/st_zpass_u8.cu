@@ -1,0 +1,304 @@
+// st_zpass_u8.cu -- the data pass on one-byte genotypes [N][2][L] (any allele count,
+// half-missing genotypes): the sweep's Z draws with counts and ln P(D), ln P(D) of a
+// state, and the Metropolis log ratios.  The initial Z, recounts, FP64 draws and
+// injected uniforms take the per-genotype kernel of st_zpass.cu; the draws here are
+// the same bits as that kernel's in FP32.
+//
+// Thread = a pair of individuals (one Philox block serves both at a locus), CTA =
+// 128 pairs x a chunk of loci whose P[l][k][.] is staged in shared memory.  Each copy
+// reads its allele's column with K loads from distinct banks (lanes differ only in
+// the allele).  Ancestry counts are lane-private columns in shared memory, allele
+// counts a histogram per CTA; both leave as one coalesced set of integer
+// reductions per CTA.  The per-genotype kernel added every copy to both
+// histograms with global atomics and took an FP64 logarithm per copy: 188 us per
+// sweep for 8 chains of N=1000, L=300, K=6, bound by those atomics' latency.
+//
+// Logarithms: a thread multiplies its copies' terms in FP64 and takes one logarithm
+// whenever the product falls below 1e-100 (terms are at least 1e-50 after
+// CalcLike's clamp, so no product underflows).
+#include "st_device.cuh"
+#include "st_kernels.h"
+#include "st_zpass_fast.cuh"
+
+namespace st {
+namespace {
+
+using zfast::block_sum_d;
+using zfast::finish_like;
+
+constexpr int kUT = 128;            // threads: pairs of individuals per CTA
+constexpr int kUMaxLc = 16;         // loci per chunk: 16-bit row counts hold 2 per locus
+constexpr size_t kUSmem = 64 * 1024;
+
+struct U8Layout { int p, n, m, total; };
+
+__host__ __device__ inline U8Layout u8_layout(int KT, int K, int A, int lc, int mode) {
+  U8Layout u;
+  int o = 0;
+  u.p = o; o += lc * KT * A * (mode == kZMetro ? 8 : 4);
+  u.n = o; if (mode == kZNormal) o += lc * K * A * 4;
+  u.m = o; if (mode == kZNormal) o += K * kUT * 4;
+  u.total = (o + 15) & ~15;
+  return u;
+}
+
+// A running product of factors and the logarithms already taken of it.
+struct LogProduct {
+  double p = 1.0, s = 0.0;
+  __device__ __forceinline__ void mul(double x) {
+    p *= x;
+    if (!(p >= 1e-100)) flush();
+  }
+  __device__ __forceinline__ void flush() {
+    s += log(p);
+    p = 1.0;
+  }
+};
+
+template <int KT, int MODE>
+__global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
+                                                 const int* __restrict__ prefix, int nchains,
+                                                 int flags) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ double sred[kUT / 32];
+  const int c = find_chain(prefix, nchains, blockIdx.x);
+  ChainDev& ch = chains[c];
+  const int tile = blockIdx.x - prefix[c];
+  const int N = ch.N, L = ch.L, K = ch.K, A = ch.A;
+  const int pb = tile / ch.u8_chunks, l0 = (tile - pb * ch.u8_chunks) * ch.u8_lc;
+  const int nl = min(ch.u8_lc, L - l0);
+  const int rep = *ch.rep;
+  const bool collect = rep + 1 > ch.burnin;
+  const bool want_like = MODE == kZLike ||
+      (MODE == kZNormal && ((flags & kZfLikeAlways) || ((flags & kZfLikeIfCollect) && collect)));
+  const U8Layout lay = u8_layout(KT, K, A, ch.u8_lc, MODE);
+  int* sN = reinterpret_cast<int*>(smem + lay.n);
+  int* sM = reinterpret_cast<int*>(smem + lay.m);
+
+  // P of the chunk's loci, [l][KT][A], zero beyond K
+  for (int idx = threadIdx.x; idx < nl * KT * A; idx += kUT) {
+    const int l = idx / (KT * A), r = idx - l * (KT * A);
+    const float v = r < K * A ? ch.P[(size_t)(l0 + l) * K * A + r] : 0.0f;
+    if (MODE == kZMetro) reinterpret_cast<double*>(smem + lay.p)[idx] = (double)v;
+    else reinterpret_cast<float*>(smem + lay.p)[idx] = v;
+  }
+  if (MODE == kZNormal) {
+    for (int idx = threadIdx.x; idx < nl * K * A; idx += kUT) sN[idx] = 0;
+    for (int k = 0; k < K; k++) sM[k * kUT + threadIdx.x] = 0;
+  }
+  __syncthreads();
+
+  const int pair = pb * kUT + threadIdx.x;
+  const int i0 = 2 * pair;
+  const int nh = min(2, N - i0);   // individuals of this thread (<= 0: none)
+  double like_acc = 0.0;
+  if constexpr (MODE == kZMetro) {
+    const double* sP = reinterpret_cast<const double*>(smem + lay.p);
+    for (int h = 0; h < nh; h++) {
+      const int i = i0 + h;
+      double q[KT], t[KT];
+#pragma unroll
+      for (int k = 0; k < KT; k++) {
+        q[k] = k < K ? (double)ch.Q[(size_t)i * K + k] : 0.0;
+        t[k] = k < K ? (double)ch.TestQ[(size_t)i * K + k] : 0.0;
+      }
+      const uint8_t* g = ch.g8 + (size_t)i * 2 * L + l0;
+      LogProduct tp, tm;
+      for (int l = 0; l < nl; l++) {
+#pragma unroll
+        for (int line = 0; line < 2; line++) {
+          const int a = g[line * L + l];
+          if (a == kG8Missing) continue;
+          const double* P = sP + l * KT * A + a;
+          double st = 0.0, sm = 0.0;
+#pragma unroll
+          for (int k = 0; k < KT; k++) {
+            const double p = P[k * A];
+            st += t[k] * p;
+            sm += q[k] * p;
+          }
+          tp.mul(st);
+          tm.mul(sm);
+        }
+      }
+      tp.flush();
+      tm.flush();
+      const double ld = tp.s - tm.s;
+      if (ld != 0.0) atomicAdd(&ch.ldpart[i], ld);
+    }
+    return;
+  } else {
+    const float* sP = reinterpret_cast<const float*>(smem + lay.p);
+    const uint32_t key = ch.key;
+    float q[2][KT];
+    bool ncnt[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+#pragma unroll
+      for (int k = 0; k < KT; k++)
+        q[h][k] = h < nh && k < K ? ch.Q[(size_t)(i0 + h) * K + k] : 0.0f;
+      ncnt[h] = h < nh && (!ch.pfrompopflagonly || ch.popflags[i0 + h] == 1);
+    }
+    const bool store_z = MODE == kZNormal && (flags & kZfStoreZ) && ch.Z;
+    LogProduct lp;
+    // rows of the pair's copies; a thread without individuals reads row 0 as missing
+    const uint8_t* g[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) g[r] = ch.g8 + (size_t)((r >> 1) < nh ? i0 * 2 + r : 0) * L + l0;
+    uint8_t nx[4];
+#pragma unroll
+    for (int r = 0; r < 4; r++) nx[r] = (r >> 1) < nh && nl > 0 ? g[r][0] : kG8Missing;
+    for (int l = 0; l < nl; l++) {
+      int a[4];
+#pragma unroll
+      for (int r = 0; r < 4; r++) {
+        a[r] = nx[r];
+        nx[r] = (r >> 1) < nh && l + 1 < nl ? g[r][l + 1] : kG8Missing;
+      }
+      U4 w{0, 0, 0, 0};
+      if (MODE == kZNormal)
+        w = philox_s((uint32_t)(l0 + l), (uint32_t)pair, (uint32_t)rep, (uint32_t)kSZ, key);
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        const bool m0 = a[2 * h] == kG8Missing, m1 = a[2 * h + 1] == kG8Missing;
+        const float* P0 = sP + l * KT * A + (m0 ? 0 : a[2 * h]);
+        const float* P1 = sP + l * KT * A + (m1 ? 0 : a[2 * h + 1]);
+        float2 C[KT];
+#pragma unroll
+        for (int k = 0; k < KT; k++) {
+          const float2 X = make_float2(P0[k * A], P1[k * A]);
+          const float2 qq = make_float2(q[h][k], q[h][k]);
+          C[k] = k == 0 ? mul2_rn(qq, X) : fma2_rn(qq, X, C[k > 0 ? k - 1 : 0]);
+        }
+        const float2 T = C[KT - 1];
+        if (want_like) {
+          if (!m0) lp.mul(fmax((double)T.x, 1e-50));
+          if (!m1) lp.mul(fmax((double)T.y, 1e-50));
+        }
+        if (MODE == kZNormal) {
+          // z = #{k : C_k < RN(u T)}: the signs of C_k - r (st_zpass_fast.cuh)
+          const float2 NM = make_float2(neg_one_plus_u23(h ? w.z : w.x),
+                                        neg_one_plus_u23(h ? w.w : w.y));
+          const float2 NR = fma2_rn(NM, T, T);
+          uint32_t t0 = 0u, t1 = 0u;
+#pragma unroll
+          for (int k = 0; k < KT - 1; k++) {
+            const float2 D = add2_rn(C[k], NR);
+            t0 = __funnelshift_l(__float_as_uint(D.x), t0, 1);
+            t1 = __funnelshift_l(__float_as_uint(D.y), t1, 1);
+          }
+          const int z0 = __popc(t0), z1 = __popc(t1), one = h ? 65536 : 1;
+          if (!m0) {
+            atomicAdd(&sM[z0 * kUT + threadIdx.x], one);
+            if (ncnt[h]) atomicAdd(&sN[(l * K + z0) * A + a[2 * h]], 1);
+          }
+          if (!m1) {
+            atomicAdd(&sM[z1 * kUT + threadIdx.x], one);
+            if (ncnt[h]) atomicAdd(&sN[(l * K + z1) * A + a[2 * h + 1]], 1);
+          }
+          if (store_z && h < nh) {
+            uint8_t* Z = ch.Z + (size_t)(i0 + h) * 2 * L + l0 + l;
+            Z[0] = m0 ? kZMissing : (uint8_t)z0;
+            Z[L] = m1 ? kZMissing : (uint8_t)z1;
+          }
+        }
+      }
+    }
+    if (want_like) {
+      lp.flush();
+      like_acc = lp.s;
+    }
+    if (MODE == kZNormal) {
+      __syncthreads();
+      for (int idx = threadIdx.x; idx < nl * K * A; idx += kUT) {   // locus fastest
+        const int ka = idx / nl, l = idx - ka * nl;
+        const int v = sN[l * K * A + ka];
+        if (v) atomicAdd(&ch.npart[(size_t)ka * L + l0 + l], v);
+      }
+      const int r0 = pb * 2 * kUT, nr = min(2 * kUT, N - r0);
+      int* dst = ch.mpart + (size_t)r0 * K;
+      for (int idx = threadIdx.x; idx < nr * K; idx += kUT) {
+        const int ii = idx / K, k = idx - ii * K;
+        const int v = (sM[k * kUT + (ii >> 1)] >> (16 * (ii & 1))) & 0xFFFF;
+        if (v) atomicAdd(&dst[idx], v);
+      }
+    }
+  }
+  const int ntiles = ch.u8_chunks * ((N + 2 * kUT - 1) / (2 * kUT));
+  if (want_like) {
+    const double s = block_sum_d(like_acc, sred);
+    if (threadIdx.x == 0) ch.likepart[tile] = s;
+  }
+  const bool advance = MODE == kZNormal && (flags & kZfAdvance) != 0;
+  if (want_like || advance) {
+    if (last_cta_arrive(&ch.ctr[kCtrZ], (unsigned)ntiles)) {
+      if (want_like) finish_like(ch, ntiles, collect && (flags & kZfCollect), sred);
+      if (advance && threadIdx.x == 0) *ch.rep = rep + 1;
+    }
+  }
+}
+
+template <int KT>
+cudaError_t launch_kt(const LaunchSet& ls, int mode, int flags, size_t smem) {
+  auto go = [&](auto fn) {
+    if (smem > 40 * 1024) {
+      const cudaError_t e =
+          cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+      if (e != cudaSuccess) return e;
+    }
+    fn<<<ls.total_ctas, kUT, smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);
+    return cudaGetLastError();
+  };
+  switch (mode) {
+    case kZNormal: return go(u8_kernel<KT, kZNormal>);
+    case kZLike: return go(u8_kernel<KT, kZLike>);
+    case kZMetro: return go(u8_kernel<KT, kZMetro>);
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace
+
+int u8_kclass(int K) {
+  for (int k : {2, 3, 4, 6, 8, 12, 16, 24, 32})
+    if (k >= K) return k;
+  return 0;
+}
+
+int ctas_u8(const ChainDev& c) { return c.u8_chunks * ((c.N + 2 * kUT - 1) / (2 * kUT)); }
+
+size_t u8_smem(const ChainDev& c, int mode) {
+  return (size_t)u8_layout(u8_kclass(c.K), c.K, c.A, c.u8_lc, mode).total;
+}
+
+// Loci per chunk: about two CTAs per SM from one chain (a small chain gets one locus
+// per CTA, a large one up to 16 so that a CTA's staging and reductions are shared by
+// more copies), within the shared memory and the room for the partials.  It depends
+// on the chain's shape alone, so ln P(D) is the same in a batch.
+int u8_plan(int N, int L, int K, int A, long cap) {
+  const long blocks = (N + 2 * kUT - 1) / (2 * kUT);
+  long lc = (L * blocks + 148 * 2 - 1) / (148 * 2);
+  if (lc > kUMaxLc) lc = kUMaxLc;
+  const int KT = u8_kclass(K);
+  while (lc > 1 && (u8_layout(KT, K, A, (int)lc, kZNormal).total > (int)kUSmem ||
+                    u8_layout(KT, K, A, (int)lc, kZMetro).total > (int)kUSmem))
+    lc--;
+  while (lc <= kUMaxLc && blocks * ((L + lc - 1) / lc) > cap) lc++;
+  if (lc > kUMaxLc || u8_layout(KT, K, A, (int)lc, kZNormal).total > 200 * 1024 ||
+      u8_layout(KT, K, A, (int)lc, kZMetro).total > 200 * 1024)
+    return 0;
+  return (int)lc;
+}
+
+// The launch's chains share the K class KT; smem: their largest u8_smem.
+cudaError_t launch_u8(const LaunchSet& ls, int KT, int mode, int flags, size_t smem) {
+  switch (KT) {
+#define ST_KCASE(k) case k: return launch_kt<k>(ls, mode, flags, smem);
+    ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(6) ST_KCASE(8) ST_KCASE(12) ST_KCASE(16)
+    ST_KCASE(24) ST_KCASE(32)
+#undef ST_KCASE
+  }
+  return cudaErrorInvalidValue;
+}
+
+}  // namespace st
