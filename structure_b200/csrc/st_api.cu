@@ -867,7 +867,7 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
     h.key = (uint32_t)z;
   }
   h.g2 = data->g2; h.g8 = data->g8; h.numalleles = data->numalleles; h.popflags = data->popflags;
-  h.loc_tpl = locus_lanes(L, K, A);
+  h.loc_tpl = locus_lanes(L, K, A, 0);
 
   c->fast = data->layout == kLayoutB2G && model->precision == 0 && fast_kt(K) > 0;
   if (data->layout == kLayoutB2G && !c->fast) {
@@ -1639,9 +1639,15 @@ static int batch_layout(st_batch* b, bool keep_groups) {
   if (!keep_groups) b->zg.clear();
   for (ZGroup& g : b->zg) { g.tz = g.tzc = 0; g.zsmem = g.zsmem_ct = 0; g.n = 0; }
   size_t gi = 0;
+  long total_loci = 0;
+  for (const st_chain* c : b->chains) total_loci += c->h.L;
   for (int j = 0; j < n; j++) {
     st_chain* c = b->chains[j];
     b->table[j] = c->h;
+    // with two alleles the lanes per locus change no bit of P (a sum of two terms),
+    // so a batch takes fewer of them; with more, every chain keeps its own
+    if (c->h.A <= 2)
+      b->table[j].loc_tpl = locus_lanes(c->h.L, c->h.K, c->h.A, total_loci - c->h.L);
     b->table[j].G = b->G;   // every chain's kernels index their groups by the batch-wide G
     if (!b->fast && b->u8) {
       if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT)) {

@@ -64,6 +64,11 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
   const int l = tile * ((int)blockDim.x / tpl) + (int)threadIdx.x / tpl;
   const int sub = (int)threadIdx.x % tpl;
   const bool lvalid = l < L && sub == 0;
+  // the lanes of a locus: population slot k0 (strided by kslots), allele slot j
+  // (strided by J)
+  int J = 1;
+  while (J * 2 * K <= tpl && J * 2 <= 32) J *= 2;
+  const int kslots = tpl / J, j = sub % J, k0 = sub / J;
   const int rep = *ch.rep;
   const uint32_t key = ch.key;
   const bool collect = (stages & kLocCollect) && (rep + 1 > ch.burnin);
@@ -81,13 +86,9 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
 
   // ---- P ------------------------------------------------------------------
   if ((stages & kLocP) && tpl > 1) {
-    // lanes (k, j) of the locus: population k (strided by tpl / J when K
-    // exceeds it), alleles a = j, j + J, ...; the Dirichlet's log-sum over the
-    // alleles of (l, k) is a width-J butterfly over contiguous lanes
-    int J = 1;
-    while (J * 2 * K <= tpl && J * 2 <= 32) J *= 2;
-    const int kslots = tpl / J;
-    const int j = sub % J, k0 = sub / J;
+    // population k (strided by tpl / J when K exceeds it), alleles a = j, j + J,
+    // ...; the Dirichlet's log-sum over the alleles of (l, k) is a width-J
+    // butterfly over contiguous lanes
     // lanes of a locus stay together through the loop: every lane runs the
     // same number of rounds
     for (int kb = 0; kb < K; kb += kslots) {
@@ -179,8 +180,8 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
                                                                (uint32_t)rep, kSP, key, &errb)
                                   : -INFINITY;
         const double M = (na > 1 && lg1 > lg0) ? lg1 : lg0;
-        double S = exp(lg0 - M);
-        if (na > 1) S += exp(lg1 - M);
+        // exp(0) = 1 for the larger one
+        const double S = na > 1 ? 1.0 + exp((lg1 > lg0 ? lg0 : lg1) - M) : 1.0;
         const double ls = M + log(S);
         emit(0, lg0, ls, na);
         if (na > 1) emit(1, lg1, ls, na);
@@ -223,53 +224,69 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
   }
 
   // ---- eps ----------------------------------------------------------------
-  if ((stages & kLocEps) && ch.freqscorr && lvalid) {
+  // The lanes of a locus share its populations (all of them idled but the first
+  // before: 140 us a sweep at 8 chains of L=300, K=6, 32 lanes per locus).
+  if ((stages & kLocEps) && ch.freqscorr) {
+    __syncwarp();   // the P stage's log P of this locus, written by its lanes
+    bool open = false;
+    int a1 = 0, a2 = 0;
+    double d = 0.0, e1 = 0.0, e2 = 0.0, sum = 0.0;
     if (na > 1) {
       const U4 w = philox_s((uint32_t)l, 0, (uint32_t)rep, kSEps, key);
-      const int a1 = (int)(((double)(w.x >> 1) / 2147483648.0) * na);
-      int a2 = (int)(((double)(w.y >> 1) / 2147483648.0) * (na - 1));
+      a1 = (int)(((double)(w.x >> 1) / 2147483648.0) * na);
+      a2 = (int)(((double)(w.y >> 1) / 2147483648.0) * (na - 1));
       if (a2 >= a1) a2 += 1;
-      const double d = 0.0 + ((double)(w.z >> 1) / 2147483648.0) * (ch.invsqrtnuminds - 0.0);
-      const double e1 = ch.eps[(size_t)l * A + a1];
-      const double e2 = ch.eps[(size_t)l * A + a2];
-      if ((e1 + d < 1.0) && (e2 - d > 0.0)) {
-        double sum = 0.0;
-        for (int k = 0; k < K; k++) {
-          const double frac = sFrac[k];
-          const size_t base = ((size_t)l * K + k) * A;
-          const double lp1 = (double)ch.logP[base + a1];
-          const double lp2 = (double)ch.logP[base + a2];
-          double s = lanczos_lgamma_fast(frac * e1);
-          s += lanczos_lgamma_fast(frac * e2);
-          s -= lanczos_lgamma_fast(frac * (e1 + d));
-          s -= lanczos_lgamma_fast(frac * (e2 - d));
-          s += frac * d * lp1;
-          s -= frac * d * lp2;
-          sum += s;
-        }
-        const double lam = ch.lambda[0];
-        if (lam != 1.0) sum += log(pow((e1 + d) * (e2 - d) / e1 / e2, lam - 1.0));
-        const U4 u = philox_s((uint32_t)l, 1, (uint32_t)rep, kSEps, key);
-        if (rnd31(u) < exp(sum)) {
-          ch.eps[(size_t)l * A + a1] = e1 + d;
-          ch.eps[(size_t)l * A + a2] = e2 - d;
-        }
+      d = 0.0 + ((double)(w.z >> 1) / 2147483648.0) * (ch.invsqrtnuminds - 0.0);
+      e1 = ch.eps[(size_t)l * A + a1];
+      e2 = ch.eps[(size_t)l * A + a2];
+      open = (e1 + d < 1.0) && (e2 - d > 0.0);
+    }
+    if (open && j == 0) {
+      for (int k = k0; k < K; k += kslots) {
+        const double frac = sFrac[k];
+        const size_t base = ((size_t)l * K + k) * A;
+        const double lp1 = (double)ch.logP[base + a1];
+        const double lp2 = (double)ch.logP[base + a2];
+        double s = lgamma_2m2(frac * e1, frac * e2, frac * (e1 + d), frac * (e2 - d));
+        s += frac * d * lp1;
+        s -= frac * d * lp2;
+        sum += s;
       }
     }
+    sum = group_sum(sum, tpl);
+    if (open && sub == 0) {
+      const double lam = ch.lambda[0];
+      if (lam != 1.0) sum += log(pow((e1 + d) * (e2 - d) / e1 / e2, lam - 1.0));
+      const U4 u = philox_s((uint32_t)l, 1, (uint32_t)rep, kSEps, key);
+      if (rnd31(u) < exp(sum)) {
+        ch.eps[(size_t)l * A + a1] = e1 + d;
+        ch.eps[(size_t)l * A + a2] = e2 - d;
+      }
+    }
+    __syncwarp();
     if (collect)
-      for (int a = 0; a < na; a++) ch.SumEps[(size_t)l * A + a] += ch.eps[(size_t)l * A + a];
+      for (int a = sub; a < na; a += tpl)
+        ch.SumEps[(size_t)l * A + a] += ch.eps[(size_t)l * A + a];
   }
 
   // ---- F ------------------------------------------------------------------
   if (fstage) {
     // per-warp sums of each proposal's locus terms, then CTA sums in warp order
     const int nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // population k's terms over this lane's alleles j, j + J, ..., in pairs
     auto fterm = [&](int k, double nf) {
       double v = 0.0;
-      if (lvalid && nf > 0.0 && nf < 1.0) {
+      if (l < L && k < K && nf > 0.0 && nf < 1.0) {
         const double nfr = (1.0 - nf) / nf, ofr = sFrac[k];
         const size_t base = ((size_t)l * K + k) * A;
-        for (int a = 0; a < na; a++) {
+        int a = j;
+        for (; a + J < na; a += 2 * J) {
+          const double e0 = ch.eps[(size_t)l * A + a], e1 = ch.eps[(size_t)l * A + a + J];
+          const double lp0 = (double)ch.logP[base + a], lp1 = (double)ch.logP[base + a + J];
+          v += (nfr - ofr) * e0 * lp0 + (nfr - ofr) * e1 * lp1 -
+               lgamma_2m2(nfr * e0, nfr * e1, ofr * e0, ofr * e1);
+        }
+        if (a < na) {
           const double e = ch.eps[(size_t)l * A + a];
           const double lp = (double)ch.logP[base + a];
           v += (nfr - ofr) * e * lp - (lanczos_lgamma_fast(nfr * e) - lanczos_lgamma_fast(ofr * e));
@@ -277,15 +294,21 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       }
       return v;
     };
-    for (int j = 0; j < numfst; j++) {
-      double v = 0.0;
+    double vone = 0.0;
+    for (int kb = 0; kb < K; kb += kslots) {
+      const int k = kb + k0;
+      double v = fterm(k, sNF[ch.onefst || k >= K ? 0 : k]);
       if (ch.onefst) {
-        for (int k = 0; k < K; k++) v += fterm(k, sNF[0]);
-      } else {
-        v = fterm(j, sNF[j]);
+        vone += v;
+      } else {   // over the allele slots and the warp's loci
+        for (int off = 1; off < J; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        for (int off = tpl; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+        if (lane < tpl && j == 0 && k < K) sF[warp * numfst + k] = v;
       }
-      for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-      if (lane == 0) sF[warp * numfst + j] = v;
+    }
+    if (ch.onefst) {
+      for (int off = 16; off > 0; off >>= 1) vone += __shfl_xor_sync(0xffffffffu, vone, off);
+      if (lane == 0) sF[warp] = vone;
     }
     __syncthreads();
     const int nblocks = (L * tpl + blockDim.x - 1) / blockDim.x;
@@ -295,34 +318,42 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       ch.redpart[(size_t)tile * numfst + threadIdx.x] = s;
     }
     if (last_cta_arrive(&ch.ctr[kCtrLocus], (unsigned)nblocks)) {
-      if (threadIdx.x < numfst) {
+      // a warp per proposal adds the CTAs' sums (one thread a proposal waited for
+      // each load in turn)
+      for (int f = warp; f < numfst; f += nwarps) {
         double s = 0.0;
-        for (int b = 0; b < nblocks; b++) s += ch.redpart[(size_t)b * numfst + threadIdx.x];
-        sTot[threadIdx.x] = s;
+#pragma unroll 4
+        for (int b = lane; b < nblocks; b += 32) s += ch.redpart[(size_t)b * numfst + f];
+        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        if (lane == 0) sTot[f] = s;
       }
       __syncthreads();
-      if (threadIdx.x == 0) {
+      if (warp == 0) {   // lane = proposal: the tests do not depend on one another
         const double m = ch.fpriormean, sd = ch.fpriorsd;
-        for (int jj = 0; jj < numfst; jj++) {
-          const double oldf = ch.F[jj];
-          const double nf = sNF[jj];
-          ch.stats[kStFstNew + jj] = nf;
-          ch.stats[kStFstDiff + jj] = sTot[jj];
-          if (!(nf > 0.0 && nf < 1.0)) { ch.stats[kStFstLpd + jj] = 0.0; continue; }
-          double lpd = (m * m / (sd * sd) - 1) * log(nf / oldf) + (oldf - nf) * m / (sd * sd);
-          const double nfr = (1.0 - nf) / nf, ofr = (1.0 - oldf) / oldf;
-          const int npops = ch.onefst ? K : 1;
-          lpd += (double)ch.Leff * npops * (lanczos_lgamma_fast(nfr) - lanczos_lgamma_fast(ofr)) + sTot[jj];
-          ch.stats[kStFstLpd + jj] = lpd;
-          bool acc = lpd >= 0.0;
-          if (!acc) acc = rnd31(philox_s((uint32_t)jj, 1, (uint32_t)rep, kSFst, key)) < exp(lpd);
+        if (lane < numfst) {
+          const double oldf = ch.F[lane];
+          const double nf = sNF[lane];
+          ch.stats[kStFstNew + lane] = nf;
+          ch.stats[kStFstDiff + lane] = sTot[lane];
+          bool acc = false;
+          if (!(nf > 0.0 && nf < 1.0)) {
+            ch.stats[kStFstLpd + lane] = 0.0;
+          } else {
+            double lpd = (m * m / (sd * sd) - 1) * log(nf / oldf) + (oldf - nf) * m / (sd * sd);
+            const double nfr = (1.0 - nf) / nf, ofr = (1.0 - oldf) / oldf;
+            const int npops = ch.onefst ? K : 1;
+            lpd += (double)ch.Leff * npops * (lanczos_lgamma_fast(nfr) - lanczos_lgamma_fast(ofr)) + sTot[lane];
+            ch.stats[kStFstLpd + lane] = lpd;
+            acc = lpd >= 0.0;
+            if (!acc) acc = rnd31(philox_s((uint32_t)lane, 1, (uint32_t)rep, kSFst, key)) < exp(lpd);
+          }
           if (acc) {
             if (ch.onefst) { for (int q = 0; q < K; q++) ch.F[q] = nf; }
-            else ch.F[jj] = nf;
+            else ch.F[lane] = nf;
           }
         }
-        if (collect)
-          for (int q = 0; q < K; q++) ch.FstSum[q] += ch.F[q];
+        __syncwarp();
+        if (collect && lane < K) ch.FstSum[lane] += ch.F[lane];
       }
     }
   } else if ((stages & kLocCollect) && collect && ch.freqscorr && tile == 0 && threadIdx.x == 0) {
@@ -372,14 +403,17 @@ cudaError_t launch_init_chain(const ChainDev& h, ChainDev* d_chain, int* d_prefi
 
 int ctas_locus(const ChainDev& c, int block) { return (c.L * c.loc_tpl + block - 1) / block; }
 
-// Lanes per locus of the locus kernel: 1 for most chains; with fewer loci
-// than about two waves of threads, up to 32 per locus (a power of two), so a
-// small chain's Dirichlet draws run in parallel over populations and alleles,
-// but no more lanes than there are (population, allele) draws to spread:
-// the lanes of a locus cover populations x alleles in powers of two.
-int locus_lanes(int L, int K, int A) {
+// Lanes per locus of the locus kernel: 1 for most chains; with fewer loci (together
+// with the other chains of the launch: `others` more) than about two waves of
+// threads, up to 32 per locus (a power of two), so a small chain's draws and log
+// ratios run in parallel over populations and alleles, but no more lanes than there
+// are (population, allele) pairs to spread: the lanes of a locus cover populations x
+// alleles in powers of two.  Lanes beyond the populations idle in the eps and F
+// stages, so a launch that fills the chip without them has one per locus (a study
+// of 40 chains, L = 5,000-20,000: 682 us a sweep with 2-8 lanes, 268 with one).
+int locus_lanes(int L, int K, int A, long others) {
   int t = 1;
-  while (t < 32 && (size_t)L * t * 2 <= (size_t)148 * 256 * 2) t *= 2;
+  while (t < 32 && ((size_t)L + others) * t * 2 <= (size_t)148 * 256 * 2) t *= 2;
   int kp = 1, ap = 1;
   while (kp < K) kp *= 2;
   while (ap < A) ap *= 2;
