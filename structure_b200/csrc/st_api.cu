@@ -107,7 +107,6 @@ struct st_batch {
   int* d_pi = nullptr;     // prefix: individual kernel
   int tz = 0, tl = 0, ti = 0;
   std::vector<ZGroup> zg;  // fast path: one Z launch per K class
-  int G = 1;
   bool fast = false;
   bool u8 = false;         // every chain takes st_zpass_u8.cu (one Z launch per K class)
   bool graphs = true;                          // replay captured sweeps
@@ -361,7 +360,7 @@ int locus(st_chain* c, int stages) {
 int ind(st_chain* c, int mode, int stages) {
   Bracket br(c->ctx, ST_K_IND);
   LaunchSet ls = single(c, ctas_ind(c->h, kBlockInd));
-  return cuda_check(c->ctx, launch_ind(ls, c->h.G, mode, stages, kBlockInd), "ind");
+  return cuda_check(c->ctx, launch_ind(ls, mode, stages, kBlockInd), "ind");
 }
 
 int check_model(st_ctx* ctx, const st_model* m) {
@@ -905,7 +904,7 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
     zctas = std::max(zctas, ctas_zpass_b2g(hs));
   }
   ChainDev hw = h;
-  hw.G = 32;  // scratch sized for the widest group a batch may impose
+  hw.G = 32;  // scratch of the widest group (the Z pass shares the region)
   const int nred = std::max(ctas_locus(hw, kBlockLoc) * K, ctas_ind(hw, kBlockInd) * (K + 1));
   if (c->count) {
     // per-CTA partials of the Z pass and of the update kernels share one region
@@ -1648,7 +1647,6 @@ static int batch_layout(st_batch* b, bool keep_groups) {
     // so a batch takes fewer of them; with more, every chain keeps its own
     if (c->h.A <= 2)
       b->table[j].loc_tpl = locus_lanes(c->h.L, c->h.K, c->h.A, total_loci - c->h.L);
-    b->table[j].G = b->G;   // every chain's kernels index their groups by the batch-wide G
     if (!b->fast && b->u8) {
       if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT)) {
         ZGroup g;
@@ -1835,7 +1833,6 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
   b->fast = c0->fast;
   b->u8 = !c0->fast;
   for (st_chain* c : b->chains) b->u8 = b->u8 && c->u8;
-  int G = 1;
   for (st_chain* c : b->chains) {
     if (c->ctx != ctx || c->fast != b->fast || c->h.metrofreq != c0->h.metrofreq ||
         c->host_rep != c0->host_rep || c->model.store_z != c0->model.store_z ||
@@ -1848,9 +1845,7 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
                     "batched chains must share the context, data path, METROFREQ, COMPUTEPROB, "
                     "NOADMIX schedule, sweep counter and Z storage");
     }
-    G = std::max(G, c->h.G);
   }
-  b->G = G;
   if (int rc = batch_layout(b, false)) {
     delete b;
     return rc;
@@ -2077,7 +2072,7 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
   if (metro) {
     {
       Bracket br(ctx, ST_K_IND);
-      ST_CUDA(ctx, launch_ind(li, b->G, kIndPropose, 0, kBlockInd));
+      ST_CUDA(ctx, launch_ind(li, kIndPropose, 0, kBlockInd));
     }
     if (!b->fast)
       for (st_chain* c : b->chains)
@@ -2091,7 +2086,7 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
       }
     }
     Bracket br(ctx, ST_K_IND);
-    ST_CUDA(ctx, launch_ind(li, b->G, kIndAccept, kIndAlpha | kIndCollect, kBlockInd));
+    ST_CUDA(ctx, launch_ind(li, kIndAccept, kIndAlpha | kIndCollect, kBlockInd));
   } else {
     // NOADMIX batches share the schedule (checked at st_batch_create)
     const int rep = c0->host_rep;
@@ -2103,10 +2098,10 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
         ST_CUDA(ctx, launch_noadmix(c->h, c->d_chain, s));
       }
       Bracket br(ctx, ST_K_IND);
-      ST_CUDA(ctx, launch_ind(li, b->G, kIndNone, astage | kIndCollect, kBlockInd));
+      ST_CUDA(ctx, launch_ind(li, kIndNone, astage | kIndCollect, kBlockInd));
     } else {
       Bracket br(ctx, ST_K_IND);
-      ST_CUDA(ctx, launch_ind(li, b->G, kIndGibbs, astage | kIndCollect, kBlockInd));
+      ST_CUDA(ctx, launch_ind(li, kIndGibbs, astage | kIndCollect, kBlockInd));
     }
   }
   for (st_chain* c : b->chains) {

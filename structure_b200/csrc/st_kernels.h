@@ -68,7 +68,7 @@ size_t u8_smem(const ChainDev& c, int mode);
 cudaError_t launch_u8(const LaunchSet& ls, int KT, int mode, int flags, size_t smem);
 int u8_kclass(int K);
 cudaError_t launch_locus(const LaunchSet& ls, int stages, int block);
-cudaError_t launch_ind(const LaunchSet& ls, int G, int mode, int stages, int block);
+cudaError_t launch_ind(const LaunchSet& ls, int mode, int stages, int block);
 cudaError_t launch_collect(const LaunchSet& ls, int block);
 cudaError_t launch_lambda(const LaunchSet& ls, int block);
 // NOADMIX: per-individual population log likelihoods and the one-hot pick
