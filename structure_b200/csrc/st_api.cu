@@ -976,7 +976,7 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
     }
     GradArgs& g = c->mcur;
     g.N = N; g.L = L; g.K = K; g.wpr = data->wpr; g.g2 = data->g2;
-    grad_plan(N, L, &g);
+    grad_plan(N, L, K, false, &g);
     for (Buf b : std::vector<Buf>{{&mQp, NK * 4}, {&mG, NK * 4}, {&mGp, NK * 4}, {&mLL, (size_t)N * 8},
                                   {&mLLp, (size_t)N * 8}, {&mTh, NK * 8}, {&mThp, NK * 8},
                                   {&mEps, (size_t)N * 4}, {&mgq, (size_t)g.lchunks * NK * 4},
@@ -2233,7 +2233,7 @@ extern "C" int st_grad_create(st_ctx* ctx, st_data* data, int maxpops, int preci
   g->fp64 = precision == 64;
   GradArgs& a = g->a;
   a.N = data->N; a.L = data->L; a.K = maxpops; a.wpr = data->wpr; a.g2 = data->g2;
-  grad_plan(a.N, a.L, &a);
+  grad_plan(a.N, a.L, a.K, g->fp64, &a);
   const size_t es = g->fp64 ? 8 : 4;
   const size_t NK = (size_t)a.N * a.K, LK2 = (size_t)a.L * a.K * 2;
   struct { void** p; size_t b; } req[] = {

@@ -20,6 +20,13 @@
 //     partials [ichunk][L][K][2].
 // Both recompute S (2K FMA per genotype) instead of exchanging it.  Finishing
 // kernels sum the partials in a fixed order and apply the softmax Jacobian.
+//
+// FP32 and FP64 have kernels of their own.  The FP32 passes were bound by issue (95
+// warp instructions per 32 genotypes, 32 of them multiply-adds; issue 77 %, FMA 44 %,
+// XU 28 %).  They now take two individuals or loci per thread, so a shared-memory read
+// serves two genotypes; FP32x2 multiply-adds over the two alleles (S_0, S_1) and
+// (w_0 P_0, w_1 P_1); a class's copy numbers from a table; one reciprocal of S_0 S_1 and
+// one logarithm per four genotypes.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -66,8 +73,8 @@ __global__ void grad_softmax_kernel(GradArgs a) {
   }
 }
 
-// FP32 uses the hardware reciprocal and logarithm (a few ulp; the gradient
-// is checked to 2e-4 of its largest entry); FP64 keeps IEEE division and log.
+// FP32 uses the hardware reciprocal and logarithm (a few ulp); FP64 keeps IEEE
+// division and log.
 __device__ __forceinline__ float div_t(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ double div_t(double a, double b) { return a / b; }
 __device__ __forceinline__ float log_t(float a) { return __logf(a); }
@@ -210,6 +217,294 @@ __global__ void __launch_bounds__(kGradBlock) grad_loc_kernel(GradArgs a) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// FP32 passes
+// ---------------------------------------------------------------------------
+// Two items (individuals or loci) per thread: 256 items per CTA.
+constexpr int k32Threads = kGradBlock / 2;
+#ifndef G32_CTAS
+#define G32_CTAS(KT) (KT <= 2 ? 6 : KT <= 4 ? 5 : KT <= 10 ? 4 : 3)
+#endif
+__host__ __device__ constexpr int g32_ctas(int KT) { return G32_CTAS(KT); }
+
+// S_0 S_1 and products of four genotype terms above this are far from FP32's range
+// ends, so their reciprocal and logarithm are as good as the factors' own; a group
+// of four genotypes below it is evaluated factor by factor (genotype_terms).
+constexpr float kG32Min = 1e-30f;
+
+__device__ __forceinline__ float frcp_approx(float x) {   // 1 ulp
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return r;
+}
+
+// Copies of allele 0 and 1 of a genotype code, as a shared-memory table.
+__device__ __forceinline__ void g32_copies(float2* t) {
+  if (threadIdx.x < 4)
+    t[threadIdx.x] = make_float2(threadIdx.x == 0 ? 2.0f : threadIdx.x == 1 ? 1.0f : 0.0f,
+                                 threadIdx.x == 2 ? 2.0f : threadIdx.x == 1 ? 1.0f : 0.0f);
+}
+
+// Weights and log-likelihood of four genotypes of one item: code e of `codes` (two
+// bits each), copies c, sums S.  LL: the log-likelihood is wanted.
+template <bool LL>
+__device__ __forceinline__ void g32_weights(uint32_t codes, const float2 (&c)[4],
+                                            const float2 (&S)[4], float2 (&w)[4], float& ll) {
+  float t[4], low, e4 = 1.0f;
+#pragma unroll
+  for (int e = 0; e < 4; e++) {
+    t[e] = S[e].x * S[e].y;
+    low = e == 0 ? t[0] : fminf(low, t[e]);
+    if (LL) {
+      // S of copy 0's allele times S of copy 1's; a missing genotype counts 1
+      const bool hi = (codes >> (2 * e + 1)) & 1u, any = (codes >> (2 * e)) & 3u;
+      const bool miss = ((codes >> (2 * e)) & 3u) == 3u;
+      const float g = (hi ? S[e].y : S[e].x) * (any ? S[e].y : S[e].x);
+      e4 *= miss ? 1.0f : g;
+    }
+  }
+  if (LL) low = fminf(low, e4);
+  if (low > kG32Min) {
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      const float r = frcp_approx(t[e]);
+      w[e] = make_float2(c[e].x * S[e].y * r, c[e].y * S[e].x * r);
+    }
+    if (LL) ll += __logf(e4);
+  } else {   // rare
+#pragma unroll
+    for (int e = 0; e < 4; e++) {
+      float l1;
+      genotype_terms<float>((codes >> (2 * e)) & 3u, S[e].x, S[e].y, w[e].x, w[e].y, l1);
+      if (LL) ll += l1;
+    }
+  }
+}
+
+// Two neighbouring individuals per thread, packed: (Q_i, Q_i+1), (S_i, S_i+1), ...
+// against P broadcast from shared memory.
+template <int KT>
+__global__ void __launch_bounds__(k32Threads, g32_ctas(KT)) grad32_ind_kernel(GradArgs a) {
+  __shared__ __align__(16) float2 sP[kLB][KT];
+  __shared__ uint32_t sW[kLB][kGradBlock / 16];
+  __shared__ float2 sC[4];
+  const int N = a.N, L = a.L, K = a.K;
+  const int i0 = blockIdx.x * kGradBlock + 2 * threadIdx.x;   // the pair shares a word
+  const float* Q = static_cast<const float*>(a.Q);
+  const float* P = static_cast<const float*>(a.P);
+  float2 q[KT], g[KT];
+#pragma unroll
+  for (int k = 0; k < KT; k++) {
+    // an individual beyond the last reads Q = (1, 0, ...): finite sums, never stored
+    float v[2];
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+      v[h] = i0 + h < N ? (k < K ? Q[(size_t)(i0 + h) * K + k] : 0.0f) : (k == 0 ? 1.0f : 0.0f);
+    q[k] = make_float2(v[0], v[1]);
+    g[k] = make_float2(0.0f, 0.0f);
+  }
+  g32_copies(sC);
+  double ll[2] = {0.0, 0.0};
+  const int l0 = blockIdx.y * a.lchunk_len;
+  const int l1 = min(L, l0 + a.lchunk_len);
+  const int wcol0 = (blockIdx.x * kGradBlock) >> 4;        // first word column of the CTA
+  const int ncol = min(kGradBlock / 16, a.wpr - wcol0);
+  const int sh = 4 * (threadIdx.x & 7), myc = threadIdx.x >> 3;
+  // the next stage's P and words wait in registers while this one is worked on
+  constexpr int kPV = (kLB * KT + k32Threads - 1) / k32Threads;
+  constexpr int kWV = kLB * (kGradBlock / 16) / k32Threads;
+  float2 pv[kPV];
+  uint32_t wv[kWV];
+  auto fetch = [&](int lb) {
+    const int nj = l1 - lb;
+#pragma unroll
+    for (int r = 0; r < kPV; r++) {
+      const int idx = threadIdx.x + r * k32Threads, j = idx / KT, k = idx - j * KT;
+      // loci beyond the chunk: P = 1 and every genotype missing
+      pv[r] = make_float2(k < K ? 1.0f : 0.0f, k < K ? 1.0f : 0.0f);
+      if (j < nj && j < kLB && k < K)
+        pv[r] = *reinterpret_cast<const float2*>(P + ((size_t)(lb + j) * K + k) * 2);
+    }
+#pragma unroll
+    for (int r = 0; r < kWV; r++) {
+      const int idx = threadIdx.x + r * k32Threads;
+      const int j = idx / (kGradBlock / 16), c = idx - j * (kGradBlock / 16);
+      wv[r] = (j < nj && c < ncol) ? __ldg(a.g2 + (size_t)(lb + j) * a.wpr + wcol0 + c)
+                                   : 0xFFFFFFFFu;
+    }
+  };
+  fetch(l0);
+  for (int lb = l0; lb < l1; lb += kLB) {
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kPV; r++) {
+      const int idx = threadIdx.x + r * k32Threads;
+      if (kLB * KT % k32Threads == 0 || idx < kLB * KT) (&sP[0][0])[idx] = pv[r];
+    }
+#pragma unroll
+    for (int r = 0; r < kWV; r++) (&sW[0][0])[threadIdx.x + r * k32Threads] = wv[r];
+    __syncthreads();
+    if (lb + kLB < l1) fetch(lb + kLB);
+    float llb[2] = {0.0f, 0.0f};
+#pragma unroll 1
+    for (int j = 0; j < kLB; j += 4) {
+      uint32_t codes[2] = {0u, 0u};
+      float2 S[2][4], c[2][4], w[2][4];   // [individual][locus]: (allele 0, allele 1)
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const uint32_t wd = sW[j + e][myc] >> sh;
+        float2 s0 = make_float2(0.0f, 0.0f), s1 = s0;
+#pragma unroll
+        for (int k = 0; k < KT; k++) {
+          const float2 p = sP[j + e][k];
+          s0 = fma2_rn(q[k], make_float2(p.x, p.x), s0);
+          s1 = fma2_rn(q[k], make_float2(p.y, p.y), s1);
+        }
+        S[0][e] = make_float2(s0.x, s1.x);
+        S[1][e] = make_float2(s0.y, s1.y);
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+          const uint32_t gt = (wd >> (2 * h)) & 3u;
+          codes[h] |= gt << (2 * e);
+          c[h][e] = sC[gt];
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; h++) g32_weights<true>(codes[h], c[h], S[h], w[h], llb[h]);
+      // read P again below instead of holding four loci of it in registers
+      asm volatile("" ::: "memory");
+#pragma unroll
+      for (int e = 0; e < 4; e++) {
+        const float2 w0 = make_float2(w[0][e].x, w[1][e].x), w1 = make_float2(w[0][e].y, w[1][e].y);
+#pragma unroll
+        for (int k = 0; k < KT; k++) {
+          const float2 p = sP[j + e][k];
+          g[k] = fma2_rn(w0, make_float2(p.x, p.x), fma2_rn(w1, make_float2(p.y, p.y), g[k]));
+        }
+      }
+    }
+    ll[0] += (double)llb[0];
+    ll[1] += (double)llb[1];
+  }
+#pragma unroll
+  for (int h = 0; h < 2; h++) {
+    const int i = i0 + h;
+    if (i < N) {
+      float* gq = static_cast<float*>(a.gqpart) + ((size_t)blockIdx.y * N + i) * K;
+#pragma unroll
+      for (int k = 0; k < KT; k++)
+        if (k < K) gq[k] = h ? g[k].y : g[k].x;
+      a.llpart[(size_t)blockIdx.y * N + i] = ll[h];
+    }
+  }
+}
+
+// Two loci per thread; Q broadcast from shared memory.
+template <int KT>
+__global__ void __launch_bounds__(k32Threads, g32_ctas(KT)) grad32_loc_kernel(GradArgs a) {
+  constexpr int IT = 2, NTH = k32Threads;
+  __shared__ __align__(16) float sQ[kIB][KT];
+  __shared__ float2 sC[4];
+  const int N = a.N, L = a.L, K = a.K;
+  const float* Q = static_cast<const float*>(a.Q);
+  const float* P = static_cast<const float*>(a.P);
+  float2 p[IT][KT], g[IT][KT];
+  const uint32_t* row[IT];
+#pragma unroll
+  for (int h = 0; h < IT; h++) {
+    const int l = blockIdx.x * kGradBlock + h * NTH + threadIdx.x;
+    const bool valid = l < L;
+    row[h] = a.g2 + (size_t)(valid ? l : 0) * a.wpr;
+#pragma unroll
+    for (int k = 0; k < KT; k++) {
+      // beyond the last locus: finite sums, never stored
+      p[h][k] = make_float2(k < K ? 1.0f : 0.0f, k < K ? 1.0f : 0.0f);
+      if (valid && k < K) p[h][k] = *reinterpret_cast<const float2*>(P + ((size_t)l * K + k) * 2);
+      g[h][k] = make_float2(0.0f, 0.0f);
+    }
+  }
+  g32_copies(sC);
+  const int i0 = blockIdx.y * a.ichunk_len;   // a multiple of 16
+  const int i1 = min(N, i0 + a.ichunk_len);
+  // the next stage's Q and the next word wait in registers while this one is worked on
+  constexpr int kQV = (kIB * KT + NTH - 1) / NTH;
+  float qv[kQV];
+  auto fetch = [&](int ib) {
+#pragma unroll
+    for (int r = 0; r < kQV; r++) {
+      const int idx = threadIdx.x + r * NTH, ii = idx / KT, k = idx - ii * KT;
+      qv[r] = ib + ii < i1 ? (k < K ? Q[(size_t)(ib + ii) * K + k] : 0.0f) : (k == 0 ? 1.0f : 0.0f);
+    }
+  };
+  uint32_t nx[IT];
+#pragma unroll
+  for (int h = 0; h < IT; h++) nx[h] = __ldg(row[h] + (i0 >> 4));
+  fetch(i0);
+  for (int ib = i0; ib < i1; ib += kIB) {
+    const int ni = min(kIB, i1 - ib);
+    __syncthreads();
+#pragma unroll
+    for (int r = 0; r < kQV; r++) {
+      const int idx = threadIdx.x + r * NTH;
+      if (kIB * KT % NTH == 0 || idx < kIB * KT) (&sQ[0][0])[idx] = qv[r];
+    }
+    __syncthreads();
+    if (ib + kIB < i1) fetch(ib + kIB);
+    for (int wj = 0; wj < ni; wj += 16) {
+      const int nh = ni - wj;   // rows beyond the chunk count as missing
+      uint32_t wd[IT];
+#pragma unroll
+      for (int h = 0; h < IT; h++) {
+        wd[h] = nx[h];
+        if (ib + wj + 16 < i1) nx[h] = __ldg(row[h] + ((ib + wj) >> 4) + 1);
+        if (nh < 16) wd[h] |= 0xFFFFFFFFu << (2 * nh);
+      }
+#pragma unroll 1
+      for (int j = 0; j < 16; j += 4) {
+        float2 S[IT][4], c[IT][4], w[IT][4];
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+#pragma unroll
+          for (int h = 0; h < IT; h++) {
+            c[h][e] = sC[(wd[h] >> (2 * e)) & 3u];
+            S[h][e] = make_float2(0.0f, 0.0f);
+          }
+#pragma unroll
+          for (int k = 0; k < KT; k++) {
+            const float q = sQ[wj + j + e][k];
+#pragma unroll
+            for (int h = 0; h < IT; h++) S[h][e] = fma2_rn(make_float2(q, q), p[h][k], S[h][e]);
+          }
+        }
+        float none = 0.0f;
+#pragma unroll
+        for (int h = 0; h < IT; h++) g32_weights<false>(wd[h] & 0xFFu, c[h], S[h], w[h], none);
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+          for (int k = 0; k < KT; k++) {
+            const float q = sQ[wj + j + e][k];
+#pragma unroll
+            for (int h = 0; h < IT; h++) g[h][k] = fma2_rn(make_float2(q, q), w[h][e], g[h][k]);
+          }
+#pragma unroll
+        for (int h = 0; h < IT; h++) wd[h] >>= 8;
+      }
+    }
+  }
+#pragma unroll
+  for (int h = 0; h < IT; h++) {
+    const int l = blockIdx.x * kGradBlock + h * NTH + threadIdx.x;
+    if (l < L) {
+      float2* gp = reinterpret_cast<float2*>(static_cast<float*>(a.gppart) +
+                                             ((size_t)blockIdx.y * L + l) * K * 2);
+#pragma unroll
+      for (int k = 0; k < KT; k++)
+        if (k < K) gp[k] = g[h][k];
+    }
+  }
+}
+
 // dll/dlogit of Q, per-individual ll, and one partial of the total per CTA.
 template <typename T>
 __global__ void __launch_bounds__(kGradBlock) grad_finish_q_kernel(GradArgs a) {
@@ -281,8 +576,13 @@ template <typename T, int KT>
 cudaError_t launch_kt(const GradArgs& a) {
   const dim3 gi((a.N + kGradBlock - 1) / kGradBlock, a.lchunks);
   const dim3 gl((a.L + kGradBlock - 1) / kGradBlock, a.ichunks);
-  grad_ind_kernel<T, KT><<<gi, kGradBlock, 0, a.stream>>>(a);
-  grad_loc_kernel<T, KT><<<gl, kGradBlock, 0, a.stream>>>(a);
+  if constexpr (sizeof(T) == 4) {
+    grad32_ind_kernel<KT><<<gi, k32Threads, 0, a.stream>>>(a);
+    grad32_loc_kernel<KT><<<gl, k32Threads, 0, a.stream>>>(a);
+  } else {
+    grad_ind_kernel<T, KT><<<gi, kGradBlock, 0, a.stream>>>(a);
+    grad_loc_kernel<T, KT><<<gl, kGradBlock, 0, a.stream>>>(a);
+  }
   return cudaGetLastError();
 }
 
@@ -293,10 +593,10 @@ cudaError_t launch_t(const GradArgs& a) {
   grad_softmax_kernel<T><<<(unsigned)nsm, kGradBlock, 0, a.stream>>>(a);
   cudaError_t e = cudaSuccess;
   switch (grad_kclass(a.K)) {
-    case 2: e = launch_kt<T, 2>(a); break;
-    case 4: e = launch_kt<T, 4>(a); break;
-    case 8: e = launch_kt<T, 8>(a); break;
-    case 16: e = launch_kt<T, 16>(a); break;
+#define ST_KCASE(k) case k: e = launch_kt<T, k>(a); break;
+    ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(5) ST_KCASE(6) ST_KCASE(8) ST_KCASE(10)
+    ST_KCASE(12) ST_KCASE(16)
+#undef ST_KCASE
     default: return cudaErrorInvalidValue;
   }
   if (e != cudaSuccess) return e;
@@ -311,7 +611,7 @@ cudaError_t launch_t(const GradArgs& a) {
 template <int KT>
 cudaError_t launch_q_kt(const GradArgs& a) {
   const dim3 gi((a.N + kGradBlock - 1) / kGradBlock, a.lchunks);
-  grad_ind_kernel<float, KT><<<gi, kGradBlock, 0, a.stream>>>(a);
+  grad32_ind_kernel<KT><<<gi, k32Threads, 0, a.stream>>>(a);
   return cudaGetLastError();
 }
 
@@ -454,10 +754,10 @@ cudaError_t launch_mala_step(const GradArgs& cur, const GradArgs& prop, const Ch
 cudaError_t launch_grad_q(const GradArgs& a) {
   cudaError_t e = cudaSuccess;
   switch (grad_kclass(a.K)) {
-    case 2: e = launch_q_kt<2>(a); break;
-    case 4: e = launch_q_kt<4>(a); break;
-    case 8: e = launch_q_kt<8>(a); break;
-    case 16: e = launch_q_kt<16>(a); break;
+#define ST_KCASE(k) case k: e = launch_q_kt<k>(a); break;
+    ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(5) ST_KCASE(6) ST_KCASE(8) ST_KCASE(10)
+    ST_KCASE(12) ST_KCASE(16)
+#undef ST_KCASE
     default: return cudaErrorInvalidValue;
   }
   if (e != cudaSuccess) return e;
@@ -468,7 +768,9 @@ cudaError_t launch_grad_q(const GradArgs& a) {
 
 int grad_kclass(int K) {
   if (K < 1 || K > kGradMaxK) return 0;
-  return K <= 2 ? 2 : K <= 4 ? 4 : K <= 8 ? 8 : 16;
+  for (int k : {2, 3, 4, 5, 6, 8, 10, 12})
+    if (K <= k) return k;
+  return 16;
 }
 
 // Chunks per pass: the smallest count c (1..cmax) whose grid takes at most
@@ -491,13 +793,12 @@ int wave_chunks(int tiles, int wave, int cmax) {
   return best;
 }
 
-// Chunking: each pass's grid sized against one wave of 4 CTAs per SM on 148
-// SMs (64 registers x 256 threads per CTA), chunks of at least 64 loci or
-// individuals so the partials stay small.
-void grad_plan(int N, int L, GradArgs* a) {
+// Chunking: each pass's grid sized against one wave of resident CTAs on 148 SMs,
+// chunks of at least 64 loci or individuals so the partials stay small.
+void grad_plan(int N, int L, int K, bool fp64, GradArgs* a) {
   const int tiles_i = (N + kGradBlock - 1) / kGradBlock;
   const int tiles_l = (L + kGradBlock - 1) / kGradBlock;
-  const int wave = 148 * 4;
+  const int wave = 148 * (fp64 ? 4 : g32_ctas(grad_kclass(K)));
   const int lch = wave_chunks(tiles_i, wave, std::max(1, std::min(64, L / 64)));
   const int llen = std::max(64, (L + lch - 1) / lch);
   a->lchunk_len = llen;
