@@ -316,6 +316,8 @@ void choose_tile(const st_model* m, int N, int L, int K, int* T, int* W, int* R)
 
 void set_count_tile(ChainDev* h, CountTile t) {
   h->ct_like_magic = zcount_like_magic(h->N, h->L);
+  h->n_sl = 1;
+  h->n_ska = h->L;
   h->ctT = t.T;
   h->ctR = t.R;
   h->ctchunks = (h->N + t.T - 1) / t.T;
@@ -327,7 +329,7 @@ bool u8_mode(int mode) { return mode == kZNormal || mode == kZLike || mode == kZ
 int zpass(st_chain* c, int mode, int flags) {
   Bracket br(c->ctx, mode == kZMetro ? ST_K_METRO : (mode == kZNormal ? ST_K_ZPASS : ST_K_OTHER));
   st_ctx* ctx = c->ctx;
-  if (mode == kZNormal || mode == kZInit || mode == kZRecount) {
+  if ((mode == kZNormal || mode == kZInit || mode == kZRecount) && !(flags & kZfCleared)) {
     ST_CUDA(ctx, cudaMemsetAsync(c->h.npart, 0, sizeof(int32_t) * (size_t)c->h.K * c->h.A * c->h.L, ctx->stream));
     ST_CUDA(ctx, cudaMemsetAsync(c->h.mpart, 0, sizeof(int32_t) * (size_t)c->h.N * c->h.K, ctx->stream));
   }
@@ -1386,12 +1388,14 @@ extern "C" int st_update_locprior(st_chain* c) {
 
 static int sweep_once(st_chain* c) {
   const int zflags = (c->h.computeprob ? kZfLikeIfCollect : 0) | kZfCollect | kZfAdvance |
-                     (c->model.store_z ? kZfStoreZ : 0);
+                     kZfCleared | (c->model.store_z ? kZfStoreZ : 0);
   // with INFERLAMBDA, lambda is updated between P and eps (src/structure.c:586-599)
-  int rc = c->h.inferlambda ? locus(c, kLocP) : locus(c, kLocP | kLocEps | kLocFst | kLocCollect);
+  // the counts' readers zero them for the Z pass
+  int rc = c->h.inferlambda ? locus(c, kLocP | kLocClear)
+                            : locus(c, kLocP | kLocEps | kLocFst | kLocCollect | kLocClear);
   if (!rc && c->h.inferlambda) rc = lambda_step(c);
   if (!rc && c->h.inferlambda) rc = locus(c, kLocEps | kLocFst | kLocCollect);
-  if (!rc) rc = update_q_impl(c, kIndAlpha | kIndCollect);
+  if (!rc) rc = update_q_impl(c, kIndAlpha | kIndCollect | kIndClear);
   if (!rc && c->h.locprior) rc = locprior_step(c);
   if (!rc && c->h.lp_admix) rc = alpha_locprior_step(c);
   if (!rc && c->h.mala && c->h.K > 1) rc = mala_step(c);

@@ -26,6 +26,7 @@ enum : int {
   kZfAdvance = 0x10,       // bump the device sweep counter at the end
   kZfF64 = 0x20,           // generic path: FP64 arithmetic (reference bit-parity)
   kZfInjected = 0x40,      // generic path: uniforms from the injected array
+  kZfCleared = 0x100,      // the count histograms are zero already
   kZfInterleave = 0x80     // fast path: the launch's chains share one data set and
                            // tile, and block b runs tile b / nchains of chain
                            // b % nchains, so the chains' CTAs over the same loci run
@@ -33,10 +34,13 @@ enum : int {
 };
 
 // Locus-kernel stages.
-enum : int { kLocP = 0x1, kLocEps = 0x2, kLocFst = 0x4, kLocCollect = 0x8 };
+// kLocClear: the P stage zeroes the allele counts that it has read, and kIndClear
+// (with the last launch of a sweep's Q update) the ancestry counts, so that the
+// sweep's Z pass needs no memsets (kZfCleared).
+enum : int { kLocP = 0x1, kLocEps = 0x2, kLocFst = 0x4, kLocCollect = 0x8, kLocClear = 0x10 };
 // Individual-kernel modes and stages.
 enum : int { kIndGibbs = 0, kIndPropose = 1, kIndAccept = 2, kIndNone = 3 };
-enum : int { kIndAlpha = 0x1, kIndCollect = 0x2 };
+enum : int { kIndAlpha = 0x1, kIndCollect = 0x2, kIndClear = 0x4 };
 
 size_t zpass_b2g_smem(int KT, int K, int T, int W, int mode);
 // CTAs of the general Z pass at its default tile for a chain of this shape

@@ -90,6 +90,22 @@ __global__ void noalloc_sum_kernel(const Head* head, const int32_t* npart, const
   }
 }
 
+// Writes the header and clears the two histograms and the error word: one launch in
+// place of a host copy and two memsets.
+__global__ void noalloc_setup_kernel(const __grid_constant__ Head hd, Head* dhead, int32_t* n,
+                                     size_t nn, int32_t* m, size_t nm, int32_t* err) {
+  static_assert(sizeof(Head) % 4 == 0, "copied by words");
+  const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  if (blockIdx.x == 0) {
+    for (int j = threadIdx.x; j < (int)(sizeof(Head) / 4); j += blockDim.x)
+      reinterpret_cast<uint32_t*>(dhead)[j] = reinterpret_cast<const uint32_t*>(&hd)[j];
+    if (err && threadIdx.x == 0) *err = 0;
+  }
+  for (size_t j = t; j < nn; j += stride) n[j] = 0;
+  for (size_t j = t; j < nm; j += stride) m[j] = 0;
+}
+
 // Device address of g_scratch on `device` (which is current), looked up once.
 int scratch_addr(int device, void** out) {
   std::lock_guard<std::mutex> lk(g_mu);
@@ -152,23 +168,31 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
   h.g2 = g2;
   h.Q = const_cast<float*>(Q);
   h.P = const_cast<float*>(P);
-  h.npart = reinterpret_cast<int32_t*>(s + o_n);
-  h.mpart = reinterpret_cast<int32_t*>(s + o_m);
+  // A small problem adds straight into the caller's arrays ([l][k][a] reductions of 4
+  // bytes here and there); a larger one into [k][a][l], where a warp's reductions
+  // coalesce, and a last kernel lays them out: its launch costs more than 2^18
+  // scattered reductions (about 2 us each way).
+  const size_t nn = (size_t)K * 2 * L, nm = (size_t)N * K;
+  const bool direct = nn * nchunks <= ((size_t)1 << 18);
+  h.npart = direct ? n_out : reinterpret_cast<int32_t*>(s + o_n);
+  h.mpart = direct ? m_out : reinterpret_cast<int32_t*>(s + o_m);
+  h.n_sl = direct ? 2 * K : 1;
+  h.n_ska = direct ? 1 : L;
   h.stats = reinterpret_cast<double*>(s + o_stats);
+  if (direct && like_out) h.stats = like_out - kStLike;   // the pass writes no other statistic
   h.likepart = reinterpret_cast<double*>(s + o_like);
   Head* dhead = reinterpret_cast<Head*>(s);
   h.ctr = dhead->ctr;
   h.rep = &dhead->rep;
-  h.err = &dhead->err;
+  h.err = direct && err_out ? err_out : &dhead->err;
   hd.rep = rep;
 
-  // pageable source: the call returns once the bytes are staged
-  if (cudaMemcpyAsync(dhead, &hd, sizeof hd, cudaMemcpyHostToDevice, stream) != cudaSuccess)
-    return ST_ERR_CUDA;
   // the Z pass adds into the histograms: they must start at zero
-  if (cudaMemsetAsync(s + o_n, 0, nbytes, stream) != cudaSuccess ||
-      cudaMemsetAsync(s + o_m, 0, mbytes, stream) != cudaSuccess)
-    return ST_ERR_CUDA;
+  size_t zblocks = ((nn > nm ? nn : nm) + 1023) / 1024;
+  if (zblocks > 148 * 4) zblocks = 148 * 4;
+  noalloc_setup_kernel<<<(unsigned)zblocks, 256, 0, stream>>>(hd, dhead, h.npart, nn, h.mpart, nm,
+                                                              direct ? err_out : nullptr);
+  if (cudaGetLastError() != cudaSuccess) return ST_ERR_CUDA;
 
   LaunchSet ls;
   ls.chains = &dhead->chain;
@@ -179,8 +203,8 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
   if (launch_zcount(ls, KT, like_out ? kZfLikeAlways : 0, zcount_smem(KT, t.T)) != cudaSuccess)
     return ST_ERR_CUDA;
 
-  const size_t total = (size_t)K * 2 * L + (size_t)N * K;
-  size_t blocks = (total + 255) / 256;
+  if (direct) return ST_OK;
+  size_t blocks = (nn + nm + 255) / 256;
   if (blocks > 148 * 8) blocks = 148 * 8;
   noalloc_sum_kernel<<<(unsigned)blocks, 256, 0, stream>>>(
       dhead, h.npart, h.mpart, h.stats, n_out, m_out, like_out, err_out);

@@ -72,6 +72,9 @@ struct ChainDev {
   // count histogram slices summed by the consumers (1: every producer adds
   // into slice 0); Metropolis log-ratio partials have ngroups slices
   int cnt_chunks, cnt_groups;
+  // where the counting Z pass adds allele counts: npart[l n_sl + (k A + a) n_ska]
+  // ([K][A][L] everywhere but in st_noalloc.cu)
+  int n_sl, n_ska;
   // tile of the counting Z pass: individuals per chunk, locus blocks per CTA, and
   // the chunks and locus groups they make
   int ctT, ctR, ctchunks, ctgroups;

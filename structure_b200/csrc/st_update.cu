@@ -101,8 +101,11 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       if (kv) {
         for (int a = j; a < na && a < kMaxAlleles; a += J) {
           int n = 0;
-          for (int cc = 0; cc < ch.cnt_chunks; cc++)
-            n += ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
+          for (int cc = 0; cc < ch.cnt_chunks; cc++) {
+            int32_t* cnt = &ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
+            n += *cnt;
+            if (stages & kLocClear) *cnt = 0;
+          }
           const double shape = ch.freqscorr ? ch.eps[(size_t)l * A + a] * sFrac[k] + (double)n
                                             : ch.lambda[k] + (double)n;
           lg[nmine] = (double)log_gamma_draw_f32((float)shape, (uint32_t)(base + a),
@@ -145,8 +148,11 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       const size_t base = ((size_t)l * K + k) * A;
       auto shape_of = [&](int a) {
         int n = 0;
-        for (int cc = 0; cc < ch.cnt_chunks; cc++)
-          n += ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
+        for (int cc = 0; cc < ch.cnt_chunks; cc++) {
+          int32_t* cnt = &ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
+          n += *cnt;
+          if (stages & kLocClear) *cnt = 0;
+        }
         // eps (1-F)/F + n (Updates/UpdateP.c:161-164), with (1-F)/F formed once per CTA
         if (ch.freqscorr) return ch.eps[(size_t)l * A + a] * sFrac[k] + (double)n;
         return ch.lambda[k] + (double)n;
@@ -599,6 +605,8 @@ ind_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nc
     qf = ch.Q[qi];
     lqf = ch.logQ[qi];
   }
+  if ((stages & kIndClear) && kvalid)
+    for (int g = 0; g < ch.cnt_groups; g++) ch.mpart[((size_t)g * N + i) * K + k] = 0;
 
   if (collect && kvalid && mode != kIndPropose) {
     ch.QSum[qi] += (double)qf;

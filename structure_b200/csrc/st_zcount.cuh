@@ -389,6 +389,7 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
 
   double like_acc = 0.0;
   const double magic = ch.ct_like_magic;
+  const int n_sl = ch.n_sl, n_ska = ch.n_ska;
   for (int rb = 0; rb < R; rb++) {
     const int lbase = ((grp * R + rb) * kW + warp) * 32;
     if (lbase >= L) break;  // warp-uniform
@@ -434,8 +435,9 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
           c1 = (d[2 * kNT] >> sft) & 0xFFFF;
         }
         const int v1 = p1 - c1, v0 = pa - ca - v1;
-        if (v0) atomicAdd(&ch.npart[((size_t)k * A + 0) * L + l], v0);
-        if (A > 1 && v1) atomicAdd(&ch.npart[((size_t)k * A + 1) * L + l], v1);
+        int32_t* dst = ch.npart + (size_t)l * n_sl + (size_t)k * A * n_ska;
+        if (v0) atomicAdd(dst, v0);
+        if (A > 1 && v1) atomicAdd(dst + n_ska, v1);
         pa = ca;
         p1 = c1;
       }
