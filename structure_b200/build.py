@@ -18,10 +18,11 @@ LIB = os.path.join(HERE, "libstgpu.so")
 SOURCES = ["st_zpass.cu", "st_zpass_u8.cu", "st_zpass_k1.cu", "st_zpass_k2.cu", "st_zpass_k3.cu",
            "st_zpass_k4.cu", "st_zpass_k5.cu", "st_zpass_k6.cu", "st_zcount_k1.cu", "st_zcount_k2.cu",
            "st_zcount_k3.cu", "st_zcount_k4.cu", "st_zcount_k5.cu", "st_zcount_k6.cu",
-           "st_zcount_k7.cu", "st_update.cu", "st_api.cu",
+           "st_zcount_k7.cu", "st_zmetro_k1.cu", "st_zmetro_k2.cu", "st_zmetro_k3.cu", "st_update.cu", "st_api.cu",
            "st_noalloc.cu", "st_grad.cu", "st_noadmix.cu",
            "st_popinfo.cu", "st_locprior.cu", "st_injected.cu"]
-HEADERS = ["st_device.cuh", "st_types.h", "st_kernels.h", "st_zpass_fast.cuh", "st_zcount.cuh"]
+HEADERS = ["st_device.cuh", "st_types.h", "st_kernels.h", "st_zpass_fast.cuh", "st_zcount.cuh",
+           "st_zmetro.cuh"]
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC",

@@ -91,7 +91,7 @@ struct ZGroup {
   int first = 0, n = 0;    // slice of the batch table
   int KT = 0, W = 8;
   bool count = false;      // counting pass (zsmem_ct, tzc, pzc) or the general one only
-  size_t zsmem = 0, zsmem_ct = 0;
+  size_t zsmem = 0, zsmem_ct = 0, msmem = 0;   // general, counting, Metropolis pass
   int tz = 0, tzc = 0;     // CTAs of the slice: general pass, counting pass
   bool same = false;       // one data set and tile for the whole slice (kZfInterleave)
 };
@@ -333,9 +333,13 @@ int zpass(st_chain* c, int mode, int flags) {
     ST_CUDA(ctx, cudaMemsetAsync(c->h.npart, 0, sizeof(int32_t) * (size_t)c->h.K * c->h.A * c->h.L, ctx->stream));
     ST_CUDA(ctx, cudaMemsetAsync(c->h.mpart, 0, sizeof(int32_t) * (size_t)c->h.N * c->h.K, ctx->stream));
   }
-  if (c->count && mode == kZNormal) {
+  if (c->count && (mode == kZNormal || mode == kZLike)) {
     LaunchSet ls = single(c, c->h.ctchunks * c->h.ctgroups);
-    return cuda_check(c->ctx, launch_zcount(ls, c->KT, flags, zcount_smem(c->KT, c->h.ctT)), "zcount");
+    return cuda_check(c->ctx, launch_zcount(ls, c->KT, mode, flags, zcount_smem(c->KT, c->h.ctT)), "zcount");
+  }
+  if (c->fast && mode == kZMetro) {
+    LaunchSet ls = single(c, ctas_zpass_b2g(c->h));
+    return cuda_check(c->ctx, launch_zmetro(ls, c->KT, flags, zmetro_smem(c->KT, c->h.tileT)), "zmetro");
   }
   if (c->fast) {
     LaunchSet ls = single(c, ctas_zpass_b2g(c->h));
@@ -1640,7 +1644,7 @@ static int batch_layout(st_batch* b, bool keep_groups) {
   b->pi.assign(n, 0);
   b->tz = b->tl = b->ti = 0;
   if (!keep_groups) b->zg.clear();
-  for (ZGroup& g : b->zg) { g.tz = g.tzc = 0; g.zsmem = g.zsmem_ct = 0; g.n = 0; }
+  for (ZGroup& g : b->zg) { g.tz = g.tzc = 0; g.zsmem = g.zsmem_ct = g.msmem = 0; g.n = 0; }
   size_t gi = 0;
   long total_loci = 0;
   for (const st_chain* c : b->chains) total_loci += c->h.L;
@@ -1662,7 +1666,7 @@ static int batch_layout(st_batch* b, bool keep_groups) {
       b->pz[j] = g.tz;
       g.tz += ctas_u8(b->table[j]);
       g.zsmem = std::max(g.zsmem, u8_smem(c->h, kZNormal));
-      g.zsmem_ct = std::max(g.zsmem_ct, u8_smem(c->h, kZMetro));
+      g.msmem = std::max(g.msmem, u8_smem(c->h, kZMetro));
       g.n++;
     } else if (b->fast) {
       if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT ||
@@ -1681,6 +1685,7 @@ static int batch_layout(st_batch* b, bool keep_groups) {
       b->pz[j] = g.tz;
       g.tz += ctas_zpass_b2g(b->table[j]);
       g.zsmem = std::max(g.zsmem, c->zsmem);
+      g.msmem = std::max(g.msmem, zmetro_smem(c->KT, c->h.tileT));
       if (g.count) {
         // a tile for the batch's CTAs together, unless one was tuned or given
         if (!c->ct_tuned)
@@ -1963,7 +1968,7 @@ extern "C" int st_batch_autotune(st_batch* b, int reps) {
         }
         cudaEventRecord(e0, s);
         const int fl = g.same ? kZfInterleave : 0;
-        cudaError_t e = g.count ? launch_zcount(lg, g.KT, fl, g.zsmem_ct)
+        cudaError_t e = g.count ? launch_zcount(lg, g.KT, kZNormal, fl, g.zsmem_ct)
                                 : launch_zpass_b2g(lg, g.KT, g.W, kZNormal, fl, g.zsmem);
         cudaEventRecord(e1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -2037,13 +2042,14 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
       const int fl = flags | (g.same ? kZfInterleave : 0);
       if (b->u8) {
         LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, gs};
-        ST_CUDA(ctx, launch_u8(lg, g.KT, mode, flags, mode == kZMetro ? g.zsmem_ct : g.zsmem));
+        ST_CUDA(ctx, launch_u8(lg, g.KT, mode, flags, mode == kZMetro ? g.msmem : g.zsmem));
       } else if (g.count && mode == kZNormal) {
         LaunchSet lg{b->d_table + g.first, b->d_pzc + g.first, g.n, g.tzc, gs};
-        ST_CUDA(ctx, launch_zcount(lg, g.KT, fl, g.zsmem_ct));
+        ST_CUDA(ctx, launch_zcount(lg, g.KT, kZNormal, fl, g.zsmem_ct));
       } else {
         LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, gs};
-        ST_CUDA(ctx, launch_zpass_b2g(lg, g.KT, g.W, mode, fl, g.zsmem));
+        ST_CUDA(ctx, mode == kZMetro ? launch_zmetro(lg, g.KT, fl, g.msmem)
+                                     : launch_zpass_b2g(lg, g.KT, g.W, mode, fl, g.zsmem));
       }
       if (fork) ST_CUDA(ctx, cudaEventRecord(b->ev_join[gi], gs));
     }

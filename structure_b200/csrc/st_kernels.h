@@ -62,7 +62,11 @@ long zcount_ctas(int N, int L, CountTile t);
 // T = 0: no tile fits.
 CountTile zcount_tile(int N, int L, int KT, int tile_t, int tile_r, int chains, long cap);
 double zcount_like_magic(int N, int L);
-cudaError_t launch_zcount(const LaunchSet& ls, int KT, int flags, size_t smem);
+// mode: kZNormal, or kZLike (ln P(D) of the state, no draws)
+cudaError_t launch_zcount(const LaunchSet& ls, int KT, int mode, int flags, size_t smem);
+// The Metropolis pass on the general pass' tile (T, R) and CTAs.
+size_t zmetro_smem(int KT, int T);
+cudaError_t launch_zmetro(const LaunchSet& ls, int KT, int flags, size_t smem);
 cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags);
 // One-byte layout, FP32 draws (st_zpass_u8.cu): modes kZNormal, kZLike and kZMetro.
 // u8_plan chooses the loci per chunk with at most `cap` CTAs; 0 if it cannot.

@@ -200,7 +200,7 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
   ls.nchains = 1;
   ls.total_ctas = (int)ntiles;
   ls.stream = stream;
-  if (launch_zcount(ls, KT, like_out ? kZfLikeAlways : 0, zcount_smem(KT, t.T)) != cudaSuccess)
+  if (launch_zcount(ls, KT, kZNormal, like_out ? kZfLikeAlways : 0, zcount_smem(KT, t.T)) != cudaSuccess)
     return ST_ERR_CUDA;
 
   if (direct) return ST_OK;

@@ -142,12 +142,14 @@ struct Locus {
   const float* Prow;
 };
 
-template <int KT, bool LIKE>
+// DRAW: draws and counts (the sweep's pass); without it ln P(D) of the state only.
+template <int KT, bool LIKE, bool DRAW>
 __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const PhiloxRun& prun,
                                              const unsigned char* xtab, const float* sQ, int* sWide,
                                              uint32_t* sRed, int* sM, int* sPres, Locus<KT>& lo,
                                              double& like_acc, double magic, int K, int A) {
-  constexpr int NT = KT - 1, NW = zc_words(KT), NS = zc_nsm(KT), KQ = zc_kq(KT);
+  constexpr int NT = DRAW ? KT - 1 : 0;
+  constexpr int NW = DRAW ? zc_words(KT) : 0, NS = zc_nsm(KT), KQ = zc_kq(KT);
   constexpr int CSTR = kNT * 8, KSTR = CSTR * zc_classes(KT);
   constexpr bool kMask = zc_classes(KT) == 3;   // missing genotypes: u = 0 instead of zero P
   constexpr int kHalves = zc_halves(KT), kJN = 16 / kHalves;
@@ -294,19 +296,21 @@ __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const P
           __syncwarp();
         }
       }
-      // present loci of the word's 16 rows, and the locus' allele totals
-      const uint32_t pres = ~(word & (word >> 1)) & 0x55555555u;
-      const uint32_t h1 = (word >> 1) & ~word & 0x55555555u;                  // 1/1
-      const uint32_t het = word & ~(word >> 1) & 0x55555555u;                 // 0/1
-      lo.tot += __popc(pres);
-      lo.tot1 += __popc(het | h1 | (h1 << 1));
-      const uint32_t q0 = __reduce_add_sync(0xffffffffu, pres & 0x01010101u);
-      const uint32_t q1 = __reduce_add_sync(0xffffffffu, (pres >> 2) & 0x01010101u);
-      const uint32_t q2 = __reduce_add_sync(0xffffffffu, (pres >> 4) & 0x01010101u);
-      const uint32_t q3 = __reduce_add_sync(0xffffffffu, (pres >> 6) & 0x01010101u);
-      if (lane < 16) {   // row 4 b + j: byte b of q_j
-        const uint32_t q = lane & 2 ? (lane & 1 ? q3 : q2) : (lane & 1 ? q1 : q0);
-        atomicAdd(&sPres[(wi << 4) + lane], (int)((q >> (8 * (lane >> 2))) & 0xFFu));
+      if constexpr (DRAW) {
+        // present loci of the word's 16 rows, and the locus' allele totals
+        const uint32_t pres = ~(word & (word >> 1)) & 0x55555555u;
+        const uint32_t h1 = (word >> 1) & ~word & 0x55555555u;                  // 1/1
+        const uint32_t het = word & ~(word >> 1) & 0x55555555u;                 // 0/1
+        lo.tot += __popc(pres);
+        lo.tot1 += __popc(het | h1 | (h1 << 1));
+        const uint32_t q0 = __reduce_add_sync(0xffffffffu, pres & 0x01010101u);
+        const uint32_t q1 = __reduce_add_sync(0xffffffffu, (pres >> 2) & 0x01010101u);
+        const uint32_t q2 = __reduce_add_sync(0xffffffffu, (pres >> 4) & 0x01010101u);
+        const uint32_t q3 = __reduce_add_sync(0xffffffffu, (pres >> 6) & 0x01010101u);
+        if (lane < 16) {   // row 4 b + j: byte b of q_j
+          const uint32_t q = lane & 2 ? (lane & 1 ? q3 : q2) : (lane & 1 ? q1 : q0);
+          atomicAdd(&sPres[(wi << 4) + lane], (int)((q >> (8 * (lane >> 2))) & 0xFFu));
+        }
       }
       if (LIKE) {
         double wl = (double)wlike;
@@ -328,7 +332,7 @@ __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const P
   }
 }
 
-template <int KT>
+template <int KT, bool DRAW>
 __global__ void __launch_bounds__(kNT, zc_ctas(KT))
 zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains, int flags) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -352,7 +356,8 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int rep = *ch.rep;
   const bool collect = rep + 1 > ch.burnin;
-  const bool want_like = (flags & kZfLikeAlways) || ((flags & kZfLikeIfCollect) && collect);
+  const bool want_like =
+      !DRAW || (flags & kZfLikeAlways) || ((flags & kZfLikeIfCollect) && collect);
 
   const ZcLayout lay = zc_layout(KT, T);
   float2* sX = reinterpret_cast<float2*>(smem + lay.x);
@@ -375,8 +380,10 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
       *reinterpret_cast<float4*>(sQ + ii * KQ + k4) = v;
     }
   }
-  for (int idx = threadIdx.x; idx < nT16 * NW * 2; idx += kNT) sM[idx] = 0;
-  for (int idx = threadIdx.x; idx < nT16; idx += kNT) sPres[idx] = 0;
+  if constexpr (DRAW) {
+    for (int idx = threadIdx.x; idx < nT16 * NW * 2; idx += kNT) sM[idx] = 0;
+    for (int idx = threadIdx.x; idx < nT16; idx += kNT) sPres[idx] = 0;
+  }
   // the zero class of the lane's table; with three classes the slot behind the
   // last one, which a missing genotype reads (finite, its draw is masked)
   if (CL == 4) {
@@ -415,15 +422,15 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
     lo.tot = lo.tot1 = 0;
     const PhiloxRun prun((uint32_t)l, (uint32_t)rep, (uint32_t)kSZ, ch.key);
 #pragma unroll
-    for (int w = 0; w < 4 * NW; w++) sWide[w * kNT] = 0;
+    for (int w = 0; w < (DRAW ? 4 * NW : 0); w++) sWide[w * kNT] = 0;
     __syncwarp();
     if (want_like)
-      zcount_words<KT, true>(nT16 >> 4, (uint32_t)(i0 >> 1), prun, smem, sQ, sWide, sRed, sM, sPres,
+      zcount_words<KT, true, DRAW>(nT16 >> 4, (uint32_t)(i0 >> 1), prun, smem, sQ, sWide, sRed, sM, sPres,
                              lo, like_acc, magic, K, A);
-    else
-      zcount_words<KT, false>(nT16 >> 4, (uint32_t)(i0 >> 1), prun, smem, sQ, sWide, sRed, sM, sPres,
+    else if constexpr (DRAW)
+      zcount_words<KT, false, true>(nT16 >> 4, (uint32_t)(i0 >> 1), prun, smem, sQ, sWide, sRed, sM, sPres,
                               lo, like_acc, magic, K, A);
-    if (valid) {
+    if (DRAW && valid) {
       // copies with C_k < r, all and of allele 1: cum_{-1} is every copy
       int pa = 2 * lo.tot, p1 = lo.tot1;
       for (int k = 0; k < K; k++) {
@@ -445,7 +452,7 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
     __syncwarp();
   }
   __syncthreads();
-  {
+  if constexpr (DRAW) {
     // thread = row: n_k = cum_{k-1} - cum_k, cum_{-1} = copies present
     for (int ii = threadIdx.x; ii < nT; ii += kNT) {
       int* dst = ch.mpart + (size_t)(i0 + ii) * K;
@@ -467,7 +474,7 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
     const double s = block_sum_d(like_acc, sred);
     if (threadIdx.x == 0) ch.likepart[tile] = s;
   }
-  const bool advance = (flags & kZfAdvance) != 0;
+  const bool advance = DRAW && (flags & kZfAdvance) != 0;
   if (want_like || advance) {
     if (last_cta_arrive(&ch.ctr[kCtrZ], (unsigned)ntiles)) {
       if (want_like) finish_like(ch, ntiles, collect && (flags & kZfCollect), sred);
@@ -477,8 +484,8 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
 }
 
 template <int KT>
-cudaError_t launch_zcount_k(const LaunchSet& ls, int flags, size_t smem) {
-  auto fn = zcount_kernel<KT>;
+cudaError_t launch_zcount_k(const LaunchSet& ls, int mode, int flags, size_t smem) {
+  auto fn = mode == kZLike ? zcount_kernel<KT, false> : zcount_kernel<KT, true>;
   if (smem > 40 * 1024) {   // above the default 48 KB with the static shared memory
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -3,7 +3,7 @@
 
 namespace st {
 namespace zcount {
-template cudaError_t launch_zcount_k<24>(const LaunchSet&, int, size_t);
-template cudaError_t launch_zcount_k<32>(const LaunchSet&, int, size_t);
+template cudaError_t launch_zcount_k<24>(const LaunchSet&, int, int, size_t);
+template cudaError_t launch_zcount_k<32>(const LaunchSet&, int, int, size_t);
 }  // namespace zcount
 }  // namespace st

@@ -93,7 +93,7 @@ cudaError_t launch_zpass_b2g(const LaunchSet& ls, int KT, int W, int mode, int f
 
 namespace zcount {
 template <int KT>
-cudaError_t launch_zcount_k(const LaunchSet& ls, int flags, size_t smem);
+cudaError_t launch_zcount_k(const LaunchSet& ls, int mode, int flags, size_t smem);
 size_t zc_layout_total(int kt, int T);
 int zc_ctas_of(int kt);
 }  // namespace zcount
@@ -167,9 +167,28 @@ double zcount_like_magic(int N, int L) {
   return ldexp(1.5, 52 - (47 - lg));
 }
 
-cudaError_t launch_zcount(const LaunchSet& ls, int KT, int flags, size_t smem) {
+cudaError_t launch_zcount(const LaunchSet& ls, int KT, int mode, int flags, size_t smem) {
   switch (KT) {
-#define ST_KCASE(k) case k: return zcount::launch_zcount_k<k>(ls, flags, smem);
+#define ST_KCASE(k) case k: return zcount::launch_zcount_k<k>(ls, mode, flags, smem);
+    ST_KCASE(1) ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(5) ST_KCASE(6) ST_KCASE(7) ST_KCASE(8)
+    ST_KCASE(9) ST_KCASE(10) ST_KCASE(11) ST_KCASE(12) ST_KCASE(16) ST_KCASE(20) ST_KCASE(24)
+    ST_KCASE(32)
+#undef ST_KCASE
+  }
+  return cudaErrorInvalidValue;
+}
+
+namespace zmetro {
+template <int KT>
+cudaError_t launch_zmetro_k(const LaunchSet& ls, int flags, size_t smem);
+size_t layout_total(int kt, int T);
+}  // namespace zmetro
+
+size_t zmetro_smem(int KT, int T) { return zmetro::layout_total(KT, T); }
+
+cudaError_t launch_zmetro(const LaunchSet& ls, int KT, int flags, size_t smem) {
+  switch (KT) {
+#define ST_KCASE(k) case k: return zmetro::launch_zmetro_k<k>(ls, flags, smem);
     ST_KCASE(1) ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(5) ST_KCASE(6) ST_KCASE(7) ST_KCASE(8)
     ST_KCASE(9) ST_KCASE(10) ST_KCASE(11) ST_KCASE(12) ST_KCASE(16) ST_KCASE(20) ST_KCASE(24)
     ST_KCASE(32)

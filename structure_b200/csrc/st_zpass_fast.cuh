@@ -124,8 +124,6 @@ struct ZArgs {
   const uint32_t* grow;
   const float2* Xlane;   // this lane's allele-table column: one pair per class and population
   const float2* sQ2;
-  const float2* sT2;
-  float* sLD;     // this warp's Metropolis log-ratio partials, one per row
   const uint2* sInc;
   int* sM;
   int* mycol;
@@ -173,37 +171,23 @@ __device__ __noinline__ double word_like_exact(uint32_t word, int row_base, cons
   return s;
 }
 
-// The Metropolis pass (no draws, no counts) is bound by the shared-memory
-// data pipe, mostly the per-lane allele-table loads; it takes the lane's
-// frequencies from registers instead (K classes up to 6, where they fit
-// without spilling).
-// The counting pass is bound by the ALU pipe, where the selects would cost
-// more than the loads.
-__host__ __device__ constexpr bool zregx(int mode, int kt) { return mode == kZMetro && kt <= 6; }
-__host__ __device__ constexpr int zregn(int mode, int kt) { return zregx(mode, kt) ? kt : 1; }
-
 // EXT: the rare per-genotype features (a stored Z, PFROMPOPFLAGONLY counts),
 // tested at run time only in this instantiation, so the common one carries
 // neither their loads nor their branches.
 template <int KT, int MODE, int W, bool LIKE, bool EXT>
-__device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, int& errb,
-                                           const float (&p0r)[zregn(MODE, KT)],
-                                           const float (&p1r)[zregn(MODE, KT)]) {
+__device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, int& errb) {
   constexpr int NW32 = 32 * W;
   constexpr int KT2 = (KT + 1) & ~1;
   constexpr int NWM = (KT + 3) / 4;
-  constexpr bool kUseP = (MODE == kZNormal || MODE == kZMetro || MODE == kZLike);
+  constexpr bool kUseP = (MODE == kZNormal || MODE == kZLike);
   constexpr bool kCounts = (MODE == kZNormal || MODE == kZInit || MODE == kZRecount);
   constexpr bool kLut = kCounts && KT <= 12;
-  constexpr bool kRegX = zregx(MODE, KT);
-  constexpr int kHalves = (zsingles(KT) && MODE != kZMetro) ? 2 : 1;
+  constexpr int kHalves = zsingles(KT) ? 2 : 1;
   constexpr int kJN = 16 / kHalves;   // genotypes of a word per unrolled pass
   ChainDev& ch = *za.chp;
   const uint32_t* grow = za.grow;
   const float2* Xlane = za.Xlane;
   const float2* sQ2 = za.sQ2;
-  const float2* sT2 = za.sT2;
-  float* sLD = za.sLD;
   const uint2* sInc = za.sInc;
   int* sM = za.sM;
   int* mycol = za.mycol;
@@ -221,7 +205,6 @@ __device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, in
       const uint32_t word = valid ? __ldg(grow + (i0 >> 4) + wi) : 0xFFFFFFFFu;
       const uint32_t pw = prun.head ^ ((uint32_t)((i0 >> 1) + (wi << 3)) & 0xFFFFFFu);
       float wlike = 0.0f, wprod = 1.0f, wmin = 1.0f;
-      float tr[MODE == kZMetro ? 16 : 1];   // Metropolis pass: this lane's term per row
       // the widest table classes walk a word in two halves of 8 genotypes, so
       // the unrolled loop body stays within the instruction cache
 #pragma unroll 1
@@ -265,19 +248,10 @@ __device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, in
                     X[k + e] = make_float2(0.0f, 0.0f);
                   }
                 }
-              } else if (!kRegX) {
+              } else {
                 // 8-byte pairs, lane-minor: a warp's load is two wavefronts
                 X[k] = X2[k * NW32];
                 X[k + 1] = k + 1 < KT ? X2[(k + 1) * NW32] : make_float2(0.0f, 0.0f);
-              }
-            }
-            if (kRegX) {
-              // (P[a0][k], P[a1][k]); a missing genotype reads class 1/1, and
-              // its terms are discarded below
-#pragma unroll
-              for (int k = 0; k < KT2; k++) {
-                const int kk = k < zregn(MODE, KT) ? k : 0;
-                X[k] = make_float2(a0 ? p1r[kk] : p0r[kk], a1 ? p1r[kk] : p0r[kk]);
               }
             }
             Cs[0] = mul2_rn(Q2[0], X[0]);
@@ -302,28 +276,6 @@ __device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, in
               }
               z0 = __popc(t0);
               z1 = __popc(t1);
-            }
-            if (MODE == kZMetro) {
-              const float4* t4 = reinterpret_cast<const float4*>(sT2 + row * KT2);
-              float2 T2[KT2];
-#pragma unroll
-              for (int k = 0; k < KT2; k += 2) {
-                const float4 v = lds_f4(t4 + (k >> 1));
-                T2[k] = make_float2(v.x, v.y);
-                T2[k + 1] = make_float2(v.z, v.w);
-              }
-              float2 S = mul2_rn(T2[0], X[0]);
-#pragma unroll
-              for (int k = 1; k < KT; k++) S = fma2_rn(T2[k], X[k], S);
-              const float tp = S.x * S.y, tm = Tp.x * Tp.y;
-              const bool tiny = !miss && !(tp > kLikeTinyF && tm > kLikeTinyF);
-              float term = miss ? 0.0f : __logf(tp) - __logf(tm);
-              if (__any_sync(0xffffffffu, tiny)) {
-                if (tiny)
-                  term = (float)(log((double)S.x) + log((double)S.y) - log((double)Tp.x) -
-                                 log((double)Tp.y));
-              }
-              tr[MODE == kZMetro ? j + h : 0] = term;
             }
             if (LIKE) {
               // j + h is a compile-time constant after unrolling
@@ -421,33 +373,6 @@ __device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, in
         }
       }
       }   // halves
-      if constexpr (MODE == kZMetro) {
-        // the word's 16 row sums over the warp's 32 loci by a transposed
-        // butterfly: at the exchange across lane bit b a lane keeps the half
-        // of its rows picked by its own bit b and adds its partner's partial
-        // for the same rows; after lane bits 4..1 lanes 2r, 2r+1 hold row r.
-        // 31 exchanges per word instead of 5 per row.
-        float v8[8], v4[4], v2[2];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          const bool hi = lane & 16;
-          v8[i] = (hi ? tr[i + 8] : tr[i]) + __shfl_xor_sync(0xffffffffu, hi ? tr[i] : tr[i + 8], 16);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-          const bool hi = lane & 8;
-          v4[i] = (hi ? v8[i + 4] : v8[i]) + __shfl_xor_sync(0xffffffffu, hi ? v8[i] : v8[i + 4], 8);
-        }
-#pragma unroll
-        for (int i = 0; i < 2; i++) {
-          const bool hi = lane & 4;
-          v2[i] = (hi ? v4[i + 2] : v4[i]) + __shfl_xor_sync(0xffffffffu, hi ? v4[i] : v4[i + 2], 4);
-        }
-        const bool hi = lane & 2;
-        float v = (hi ? v2[1] : v2[0]) + __shfl_xor_sync(0xffffffffu, hi ? v2[0] : v2[1], 2);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        if (!(lane & 1)) sLD[(wi << 4) + (lane >> 1)] += v;   // this warp's rows only
-      }
       if (LIKE) {
         double wl = (double)wlike;
         if (__any_sync(0xffffffffu, !(wmin > kLikeFastMin))) {   // once per word, rare
@@ -468,7 +393,7 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
   constexpr int NW32 = 32 * W;
   constexpr int KT2 = (KT + 1) & ~1;
   constexpr int NWM = (KT + 3) / 4;
-  constexpr bool kUseP = (MODE == kZNormal || MODE == kZMetro || MODE == kZLike);
+  constexpr bool kUseP = (MODE == kZNormal || MODE == kZLike);
   constexpr bool kCounts = (MODE == kZNormal || MODE == kZInit || MODE == kZRecount);
   constexpr bool kLut = kCounts && KT <= 12;
 
@@ -499,9 +424,7 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
 
   const ZLayout lay = zlayout(KT, K, T, NW32, MODE);
   float2* sQ2 = reinterpret_cast<float2*>(smem + lay.q2);
-  float2* sT2 = reinterpret_cast<float2*>(smem + lay.t2);
   float2* sX = reinterpret_cast<float2*>(smem + lay.x);
-  float* sLD = reinterpret_cast<float*>(smem + lay.ld);   // [W][nT16]
   uint2* sInc = reinterpret_cast<uint2*>(smem + lay.inc);
   int* sM = reinterpret_cast<int*>(smem + lay.m);
   int* sN = reinterpret_cast<int*>(smem + lay.n);
@@ -512,10 +435,6 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
       const bool in = ii < nT && k < K;
       const float q = in ? ch.Q[(size_t)(i0 + ii) * K + k] : 0.0f;
       sQ2[idx] = make_float2(q, q);
-      if (MODE == kZMetro) {
-        const float t = in ? ch.TestQ[(size_t)(i0 + ii) * K + k] : 0.0f;
-        sT2[idx] = make_float2(t, t);
-      }
     }
   }
   if (kCounts)
@@ -533,8 +452,6 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
       else reinterpret_cast<uint4*>(sInc)[idx] = make_uint4(w0, w1, field(za, 2) + field(zb, 2), 0u);
     }
   }
-  if (MODE == kZMetro)
-    for (int idx = threadIdx.x; idx < nT16 * W; idx += NW32) sLD[idx] = 0.0f;
   __syncthreads();
 
   // lane k < K extracts population k's field from the reduced words
@@ -555,10 +472,6 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
     if (lbase >= L) break;  // warp-uniform
     const int l = lbase + lane;
     const bool valid = l < L;
-    constexpr int NP = zregn(MODE, KT);
-    float p0r[NP], p1r[NP];   // Metropolis pass: this lane's P[l][k][0], P[l][k][1]
-#pragma unroll
-    for (int k = 0; k < NP; k++) p0r[k] = p1r[k] = 0.0f;
     if (kUseP) {
       // allele table of this lane's locus: for class g in {0/0, 0/1, 1/1} and
       // population k the pair (P[a0][k], P[a1][k]) at [g][k][lane], 8 bytes per
@@ -574,10 +487,6 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
           const int kk = k + e;
           p0[e] = (valid && kk < K) ? ch.P[((size_t)l * K + kk) * A] : 0.0f;
           p1[e] = (valid && kk < K && A > 1) ? ch.P[((size_t)l * K + kk) * A + 1] : 0.0f;
-          if (zregx(MODE, KT) && kk < NP) {
-            p0r[kk < NP ? kk : 0] = p0[e];
-            p1r[kk < NP ? kk : 0] = p1[e];
-          }
         }
         if (zsingles(KT)) {
           float2* XSw = reinterpret_cast<float2*>(sX) + threadIdx.x;
@@ -601,20 +510,20 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
     const uint32_t* grow = ch.g2 + (size_t)(valid ? l : 0) * ch.wpr;
     const float2* Xlane = reinterpret_cast<const float2*>(sX) + threadIdx.x;
     {
-      ZArgs za{&ch, grow, Xlane, sQ2, sT2, sLD + warp * nT16, sInc, sM, mycol, i0, i1, nT16, l,
+      ZArgs za{&ch, grow, Xlane, sQ2, sInc, sM, mycol, i0, i1, nT16, l,
                K, L, lane,
                my_word, my_shift, prep, key, stream, valid, pfonly, store_z};
       [[maybe_unused]] const bool ext = store_z || pfonly;
       if constexpr (MODE == kZNormal) {
         // chains with neither feature take the counting pass of st_zcount.cuh
-        if (want_like) zword_loop<KT, MODE, W, true, true>(za, like_acc, errb, p0r, p1r);
-        else zword_loop<KT, MODE, W, false, true>(za, like_acc, errb, p0r, p1r);
+        if (want_like) zword_loop<KT, MODE, W, true, true>(za, like_acc, errb);
+        else zword_loop<KT, MODE, W, false, true>(za, like_acc, errb);
       } else if (want_like) {
-        if (ext) zword_loop<KT, MODE, W, true, true>(za, like_acc, errb, p0r, p1r);
-        else zword_loop<KT, MODE, W, true, false>(za, like_acc, errb, p0r, p1r);
+        if (ext) zword_loop<KT, MODE, W, true, true>(za, like_acc, errb);
+        else zword_loop<KT, MODE, W, true, false>(za, like_acc, errb);
       } else {
-        if (ext) zword_loop<KT, MODE, W, false, true>(za, like_acc, errb, p0r, p1r);
-        else zword_loop<KT, MODE, W, false, false>(za, like_acc, errb, p0r, p1r);
+        if (ext) zword_loop<KT, MODE, W, false, true>(za, like_acc, errb);
+        else zword_loop<KT, MODE, W, false, false>(za, like_acc, errb);
       }
     }
     if (kCounts) {
@@ -637,15 +546,6 @@ zpass_b2g_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix,
       const int ii = idx / K;
       const int v = sM[ii * KT + (idx - ii * K)];
       if (v) atomicAdd(&dst[idx], v);
-    }
-  }
-  if (MODE == kZMetro) {
-    // the warps' partials in warp order: a fixed summation order
-    double* dst = ch.ldpart + (size_t)grp * N + i0;
-    for (int idx = threadIdx.x; idx < nT; idx += NW32) {
-      double v = 0.0;
-      for (int w = 0; w < W; w++) v += (double)sLD[w * nT16 + idx];
-      dst[idx] = v;
     }
   }
   if (errb) set_err(ch.err, errb);
@@ -679,7 +579,6 @@ cudaError_t launch_b2g_kw(const LaunchSet& ls, int mode, int flags, size_t smem)
     ST_ZCASE(kZNormal)
     ST_ZCASE(kZInit)
     ST_ZCASE(kZRecount)
-    ST_ZCASE(kZMetro)
     ST_ZCASE(kZLike)
 #undef ST_ZCASE
   }
