@@ -249,6 +249,14 @@ _DT = {F_Q: np.float32, F_LOGQ: np.float32, F_TESTQ: np.float32, F_LOGTESTQ: np.
        F_LOCPRIOR: np.float64, F_SUMLOCPRIOR: np.float64, F_MYLOC: np.int32}
 
 
+# shapes of the fields that are not flat, by the chain's dimensions
+_SHAPES = {F_Q: "NK", F_LOGQ: "NK", F_TESTQ: "NK", F_LOGTESTQ: "NK", F_P: "LKA", F_LOGP: "LKA",
+           F_EPS: "LA", F_SUMEPS: "LA", F_Z: ("N", 2, "L"), F_N: "LKA", F_M: "NK", F_LOGDIFF: "N",
+           F_QSUM: "NK", F_PSUM: "LKA", F_STATS: (256,), F_DIMS: (8,), F_MALA_EPS: "N",
+           F_USEPOPPROBS: ("N", "K", -1)}
+_NP_DT = {f: np.dtype(t) for f, t in _DT.items()}
+
+
 class Chain:
     """One MCMC chain; methods mirror the reference's *CL update twins."""
 
@@ -260,30 +268,28 @@ class Chain:
         self.N, self.L, self.K, self.A, self.layout, self.G, self.nchunks, self.ngroups = map(int, dims)
 
     def _shape(self, f):
-        N, L, K, A = self.N, self.L, self.K, self.A
-        return {F_Q: (N, K), F_LOGQ: (N, K), F_TESTQ: (N, K), F_LOGTESTQ: (N, K),
-                F_P: (L, K, A), F_LOGP: (L, K, A), F_EPS: (L, A), F_SUMEPS: (L, A),
-                F_Z: (N, 2, L), F_N: (L, K, A), F_M: (N, K), F_LOGDIFF: (N,),
-                F_QSUM: (N, K), F_PSUM: (L, K, A), F_STATS: (256,), F_DIMS: (8,),
-                F_MALA_EPS: (N,), F_USEPOPPROBS: (N, K, -1)}.get(f, None)
+        rows = _SHAPES.get(f)
+        return tuple(getattr(self, r) if isinstance(r, str) else r for r in rows) if rows else None
 
     def get(self, f, out=None):
         """Copy field f to the host.  `out`, if given, is a C-contiguous array of
         the field's type and size (page-locked memory makes the copy a direct DMA)
         and is filled and returned in the field's shape."""
         n = lib().st_field_bytes(self.h, f)
+        dt = _NP_DT[f]
         if out is None:
-            out = np.zeros(n // np.dtype(_DT[f]).itemsize, _DT[f])
-        elif (out.dtype != np.dtype(_DT[f]) or out.nbytes != n
-              or not out.flags["C_CONTIGUOUS"]):
+            out = np.zeros(n // dt.itemsize, dt)
+        elif out.dtype != dt or out.nbytes != n or not out.flags.c_contiguous:
             raise StError(ST_ERR_ARG, "field %d: output array must be C-contiguous %s of %d bytes"
-                          % (f, np.dtype(_DT[f]).name, n))
+                          % (f, dt.name, n))
         self.ctx.check(lib().st_get_state(self.h, f, out.ctypes.data, n))
-        shp = self._shape(f) if f != F_DIMS else (8,)
+        if f == F_DIMS:
+            return out.reshape(8)
         if f == F_ANCESTDIST:
             return out.reshape(self.N, self.K, -1)
         if f in (F_REP, F_ERR):
             return int(out[0])
+        shp = self._shape(f)
         return out.reshape(shp) if shp else out
 
     def set(self, f, arr):

@@ -1523,10 +1523,20 @@ extern "C" int st_get_state(st_chain* c, int f, void* host, size_t bytes) {
     return seterr(c->ctx, ST_ERR_ARG, "field %d: %zu bytes given, %zu expected", f, bytes, need);
   cudaSetDevice(c->ctx->device);
   cudaStream_t s = c->ctx->stream;
-  ST_CUDA(c->ctx, cudaStreamSynchronize(s));
   const ChainDev& h = c->h;
-  if (f == ST_F_REP) { memcpy(host, &c->host_rep, 4); return ST_OK; }
-  if (f == ST_F_DIMS) {
+  // a copy behind the chain's work on its stream and one wait (a wait, then a copy on
+  // the default stream, took 17 us per field instead of 11)
+  auto read = [&](void* to, const void* from, size_t n) -> int {
+    ST_CUDA(c->ctx, cudaMemcpyAsync(to, from, n, cudaMemcpyDeviceToHost, s));
+    ST_CUDA(c->ctx, cudaStreamSynchronize(s));
+    return ST_OK;
+  };
+  if (f == ST_F_REP || f == ST_F_DIMS) {
+    ST_CUDA(c->ctx, cudaStreamSynchronize(s));
+    if (f == ST_F_REP) {
+      memcpy(host, &c->host_rep, 4);
+      return ST_OK;
+    }
     // the tile of the sweep's Z pass
     int32_t d[8] = {h.N, h.L, h.K, h.A, h.layout, h.G, c->count ? h.ctchunks : h.nchunks,
                     c->count ? h.ctgroups : h.ngroups};
@@ -1534,23 +1544,23 @@ extern "C" int st_get_state(st_chain* c, int f, void* host, size_t bytes) {
     return ST_OK;
   }
   if (f == ST_F_N) {
-    const size_t LKA = (size_t)h.L * h.K * h.A;
-    std::vector<int32_t> part((size_t)h.cnt_chunks * LKA);
-    ST_CUDA(c->ctx, cudaMemcpy(part.data(), h.npart, part.size() * 4, cudaMemcpyDeviceToHost));
+    // [k][a][l] on the device; rows of [l] are written in order
+    const size_t KA = (size_t)h.K * h.A, L = (size_t)h.L;
+    std::vector<int32_t> part((size_t)h.cnt_chunks * L * KA);
+    if (int rc = read(part.data(), h.npart, part.size() * 4)) return rc;
     int32_t* o = (int32_t*)host;
-    memset(o, 0, bytes);
-    for (int cc = 0; cc < h.cnt_chunks; cc++)
-      for (int k = 0; k < h.K; k++)
-        for (int a = 0; a < h.A; a++)
-          for (int l = 0; l < h.L; l++)
-            o[((size_t)l * h.K + k) * h.A + a] +=
-                part[(((size_t)cc * h.K + k) * h.A + a) * h.L + l];
+    for (size_t l = 0; l < L; l++)
+      for (size_t ka = 0; ka < KA; ka++) {
+        int32_t v = 0;
+        for (int cc = 0; cc < h.cnt_chunks; cc++) v += part[(cc * KA + ka) * L + l];
+        o[l * KA + ka] = v;
+      }
     return ST_OK;
   }
-  if (f == ST_F_M) {
+  if (f == ST_F_M && h.cnt_groups > 1) {
     const size_t NK = (size_t)h.N * h.K;
     std::vector<int32_t> part((size_t)h.cnt_groups * NK);
-    ST_CUDA(c->ctx, cudaMemcpy(part.data(), h.mpart, part.size() * 4, cudaMemcpyDeviceToHost));
+    if (int rc = read(part.data(), h.mpart, part.size() * 4)) return rc;
     int32_t* o = (int32_t*)host;
     memset(o, 0, bytes);
     for (int g = 0; g < h.cnt_groups; g++)
@@ -1559,7 +1569,7 @@ extern "C" int st_get_state(st_chain* c, int f, void* host, size_t bytes) {
   }
   if (f == ST_F_LOGDIFF) {
     std::vector<double> part((size_t)h.ngroups * h.N);
-    ST_CUDA(c->ctx, cudaMemcpy(part.data(), h.ldpart, part.size() * 8, cudaMemcpyDeviceToHost));
+    if (int rc = read(part.data(), h.ldpart, part.size() * 8)) return rc;
     double* o = (double*)host;
     for (int i = 0; i < h.N; i++) {
       double s2 = 0.0;
@@ -1568,10 +1578,12 @@ extern "C" int st_get_state(st_chain* c, int f, void* host, size_t bytes) {
     }
     return ST_OK;
   }
-  void* p = field_ptr(c, f);
-  if (!p) return seterr(c->ctx, ST_ERR_STATE, "field %d not held (store_z / ancestdist off?)", f);
-  ST_CUDA(c->ctx, cudaMemcpy(host, p, bytes, cudaMemcpyDeviceToHost));
-  return ST_OK;
+  void* p = f == ST_F_M ? (void*)h.mpart : field_ptr(c, f);
+  if (!p) {
+    ST_CUDA(c->ctx, cudaStreamSynchronize(s));
+    return seterr(c->ctx, ST_ERR_STATE, "field %d not held (store_z / ancestdist off?)", f);
+  }
+  return read(host, p, bytes);
 }
 
 extern "C" int st_set_state(st_chain* c, int f, const void* host, size_t bytes) {
