@@ -709,7 +709,7 @@ extern "C" int st_data_upload(st_ctx* ctx, const st_data_desc* d, st_data** out)
     for (size_t off = 0; off < n; off += slice) {
       size_t m = std::min(slice, n - off);
       cudaMemcpy(tmp, d->geno + off, sizeof(int32_t) * m, cudaMemcpyHostToDevice);
-      launch_pack_u8(tmp, s->g8 + off, m, 0);
+      launch_pack_u8(tmp, s->g8, off, m, N, L, 0);
       ctx->launches++;
     }
     cudaDeviceSynchronize();

@@ -101,8 +101,8 @@ __global__ void __launch_bounds__(kNaBlock) noadmix_ll_u8_kernel(const ChainDev*
   const int l0 = blockIdx.y * ch.na_lchunk_len;
   const int l1 = min(L, l0 + ch.na_lchunk_len);
   for (int l = l0; l < l1; l++) {
-    const uint8_t b0 = __ldg(ch.g8 + ((size_t)i * 2) * L + l);
-    const uint8_t b1 = __ldg(ch.g8 + ((size_t)i * 2 + 1) * L + l);
+    const uint8_t b0 = __ldg(ch.g8 + ((size_t)l * N + i) * 2);
+    const uint8_t b1 = __ldg(ch.g8 + ((size_t)l * N + i) * 2 + 1);
     const int a0 = b0 == kG8Missing ? -1 : b0, a1 = b1 == kG8Missing ? -1 : b1;
     const float* lp = ch.logP + (size_t)l * K * A;
 #pragma unroll

@@ -54,8 +54,8 @@ __global__ void __launch_bounds__(kPiBlock) popinfo_ll_kernel(const ChainDev* __
         a0 = (int)(gt >> 1);
         a1 = (int)((gt | (gt >> 1)) & 1u);
       } else {
-        const uint8_t b0 = __ldg(ch.g8 + ((size_t)i * 2) * L + l);
-        const uint8_t b1 = __ldg(ch.g8 + ((size_t)i * 2 + 1) * L + l);
+        const uint8_t b0 = __ldg(ch.g8 + ((size_t)l * N + i) * 2);
+        const uint8_t b1 = __ldg(ch.g8 + ((size_t)l * N + i) * 2 + 1);
         a0 = b0 == kG8Missing ? -1 : b0;
         a1 = b1 == kG8Missing ? -1 : b1;
         if (a0 < 0 && a1 < 0) continue;

@@ -29,7 +29,7 @@ enum : int {
 
 // Genotype layouts on the device.
 enum Layout : int {
-  kLayoutU8 = 0,   // [N][2][L] bytes, allele code or 0xFF (reference order)
+  kLayoutU8 = 0,   // [L][N][2] bytes, allele code or 0xFF: individuals side by side
   kLayoutB2G = 1   // [L][wpr] uint32, 16 genotypes/word, 2 bits each:
                    // 0 = 0/0, 1 = 0/1, 2 = 1/1, 3 = missing
 };

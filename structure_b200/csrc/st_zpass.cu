@@ -262,7 +262,8 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
   double like_acc = 0.0;
 
   if (active) {
-    const uint8_t gv[2] = {ch.g8[((size_t)i * 2) * L + l], ch.g8[((size_t)i * 2 + 1) * L + l]};
+    const uint8_t* g = ch.g8 + ((size_t)l * N + i) * 2;
+    const uint8_t gv[2] = {g[0], g[1]};
     const float* q = ch.Q + (size_t)i * K;
     const float* Pl = ch.P + (size_t)l * K * A;
     U4 r4 = {0, 0, 0, 0};
@@ -344,19 +345,23 @@ cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags) {
   return cudaGetLastError();
 }
 
-// int32 reference genotypes (-9 missing) -> one byte per copy (0xFF missing).
-__global__ void pack_u8_kernel(const int32_t* __restrict__ geno, uint8_t* __restrict__ g8, size_t n) {
+// int32 reference genotypes [N][2][L] (-9 missing), elements off .. off + n - 1, to one
+// byte per copy (0xFF missing) in [L][N][2].
+__global__ void pack_u8_kernel(const int32_t* __restrict__ geno, uint8_t* __restrict__ g8, size_t off,
+                               size_t n, int N, int L) {
   for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n;
        j += (size_t)gridDim.x * blockDim.x) {
     const int v = geno[j];
-    g8[j] = (v < 0 || v > 254) ? kG8Missing : (uint8_t)v;
+    const size_t row = (off + j) / L, l = off + j - row * L;   // row = 2 i + line
+    g8[l * (size_t)N * 2 + row] = (v < 0 || v > 254) ? kG8Missing : (uint8_t)v;
   }
 }
 
-cudaError_t launch_pack_u8(const int32_t* geno, uint8_t* g8, size_t n, cudaStream_t s) {
+cudaError_t launch_pack_u8(const int32_t* geno, uint8_t* g8, size_t off, size_t n, int N, int L,
+                           cudaStream_t s) {
   int blocks = (int)((n + 255) / 256);
   if (blocks > 148 * 16) blocks = 148 * 16;
-  pack_u8_kernel<<<blocks, 256, 0, s>>>(geno, g8, n);
+  pack_u8_kernel<<<blocks, 256, 0, s>>>(geno, g8, off, n, N, L);
   return cudaGetLastError();
 }
 

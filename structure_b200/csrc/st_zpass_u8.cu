@@ -1,13 +1,17 @@
-// st_zpass_u8.cu -- the data pass on one-byte genotypes [N][2][L] (any allele count,
+// st_zpass_u8.cu -- the data pass on one-byte genotypes [L][N][2] (any allele count,
 // half-missing genotypes): the sweep's Z draws with counts and ln P(D), ln P(D) of a
 // state, and the Metropolis log ratios.  The initial Z, recounts, FP64 draws and
 // injected uniforms take the per-genotype kernel of st_zpass.cu; the draws here are
 // the same bits as that kernel's in FP32.
 //
+// The layout puts individuals side by side, so that a warp reads the copies of 32 pairs
+// at a locus as one piece ([N][2][L] took a sector per byte: 56 instead of 37 us).
 // Thread = a pair of individuals (one Philox block serves both at a locus), CTA =
-// 128 pairs x a chunk of loci whose P[l][k][.] is staged in shared memory.  Each copy
-// reads its allele's column with K loads from distinct banks (lanes differ only in
-// the allele).  Ancestry counts are lane-private columns in shared memory, allele
+// 128 pairs x a chunk of loci whose P is staged in shared memory allele by allele,
+// rows of an odd length: a copy reads its allele's row at fixed offsets, and lanes with
+// different alleles meet different banks.  Missing copies are counted as 0 or into a
+// spare slot, so that the loop has no branch but the rare logarithm (with branches and
+// rows [k][a] it took 647 warp instructions per 32 pairs and locus, 58 us).  Ancestry counts are lane-private columns in shared memory, allele
 // counts a histogram per CTA; both leave as one coalesced set of integer
 // reductions per CTA.  The per-genotype kernel added every copy to both
 // histograms with global atomics and took an FP64 logarithm per copy: 188 us per
@@ -27,16 +31,18 @@ using zfast::block_sum_d;
 using zfast::finish_like;
 
 constexpr int kUT = 128;            // threads: pairs of individuals per CTA
-constexpr int kUMaxLc = 16;         // loci per chunk: 16-bit row counts hold 2 per locus
+constexpr int kUMaxLc = 16;         // loci per chunk at most
 constexpr size_t kUSmem = 64 * 1024;
 
 struct U8Layout { int p, n, m, total; };
 
+__host__ __device__ constexpr int u8_row(int KT) { return KT | 1; }   // words of an allele's row
+
 __host__ __device__ inline U8Layout u8_layout(int KT, int K, int A, int lc, int mode) {
   U8Layout u;
   int o = 0;
-  u.p = o; o += lc * KT * A * (mode == kZMetro ? 8 : 4);
-  u.n = o; if (mode == kZNormal) o += lc * K * A * 4;
+  u.p = o; o += lc * u8_row(KT) * A * (mode == kZMetro ? 8 : 4);
+  u.n = o; if (mode == kZNormal) o += (lc * K * A + 1) * 4;   // and a spare slot
   u.m = o; if (mode == kZNormal) o += K * kUT * 4;
   u.total = (o + 15) & ~15;
   return u;
@@ -56,7 +62,7 @@ struct LogProduct {
 };
 
 template <int KT, int MODE>
-__global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
+__global__ void __launch_bounds__(kUT, KT <= 8 ? 4 : 3) u8_kernel(ChainDev* __restrict__ chains,
                                                  const int* __restrict__ prefix, int nchains,
                                                  int flags) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -75,12 +81,17 @@ __global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
   int* sN = reinterpret_cast<int*>(smem + lay.n);
   int* sM = reinterpret_cast<int*>(smem + lay.m);
 
-  // P of the chunk's loci, [l][KT][A], zero beyond K
-  for (int idx = threadIdx.x; idx < nl * KT * A; idx += kUT) {
-    const int l = idx / (KT * A), r = idx - l * (KT * A);
-    const float v = r < K * A ? ch.P[(size_t)(l0 + l) * K * A + r] : 0.0f;
-    if (MODE == kZMetro) reinterpret_cast<double*>(smem + lay.p)[idx] = (double)v;
-    else reinterpret_cast<float*>(smem + lay.p)[idx] = v;
+  // P of the chunk's loci, [l][A][KS], zero beyond K
+  constexpr int KS = u8_row(KT);
+  for (int la = threadIdx.x; la < nl * A; la += kUT) {
+    const int l = la / A, a = la - l * A;
+    const float* P = ch.P + (size_t)(l0 + l) * K * A + a;
+#pragma unroll
+    for (int k = 0; k < KT; k++) {
+      const float v = k < K ? P[(size_t)k * A] : 0.0f;
+      if (MODE == kZMetro) reinterpret_cast<double*>(smem + lay.p)[la * KS + k] = (double)v;
+      else reinterpret_cast<float*>(smem + lay.p)[la * KS + k] = v;
+    }
   }
   if (MODE == kZNormal) {
     for (int idx = threadIdx.x; idx < nl * K * A; idx += kUT) sN[idx] = 0;
@@ -102,18 +113,19 @@ __global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
         q[k] = k < K ? (double)ch.Q[(size_t)i * K + k] : 0.0;
         t[k] = k < K ? (double)ch.TestQ[(size_t)i * K + k] : 0.0;
       }
-      const uint8_t* g = ch.g8 + (size_t)i * 2 * L + l0;
+      const uint16_t* g = reinterpret_cast<const uint16_t*>(ch.g8) + (size_t)l0 * N + i;
       LogProduct tp, tm;
       for (int l = 0; l < nl; l++) {
+        const uint32_t ab = __ldg(g + (size_t)l * N);
 #pragma unroll
         for (int line = 0; line < 2; line++) {
-          const int a = g[line * L + l];
+          const int a = (int)((ab >> (8 * line)) & 0xFFu);
           if (a == kG8Missing) continue;
-          const double* P = sP + l * KT * A + a;
+          const double* P = sP + (l * A + a) * KS;
           double st = 0.0, sm = 0.0;
 #pragma unroll
           for (int k = 0; k < KT; k++) {
-            const double p = P[k * A];
+            const double p = P[k];
             st += t[k] * p;
             sm += q[k] * p;
           }
@@ -140,40 +152,46 @@ __global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
       ncnt[h] = h < nh && (!ch.pfrompopflagonly || ch.popflags[i0 + h] == 1);
     }
     const bool store_z = MODE == kZNormal && (flags & kZfStoreZ) && ch.Z;
+    const int spare = nl * K * A, KA = K * A;
+    int* myM = sM + threadIdx.x;
     LogProduct lp;
-    // rows of the pair's copies; a thread without individuals reads row 0 as missing
-    const uint8_t* g[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) g[r] = ch.g8 + (size_t)((r >> 1) < nh ? i0 * 2 + r : 0) * L + l0;
-    uint8_t nx[4];
-#pragma unroll
-    for (int r = 0; r < 4; r++) nx[r] = (r >> 1) < nh && nl > 0 ? g[r][0] : kG8Missing;
+    // the pair's copies at a locus: two 16-bit loads side by side; individuals beyond
+    // the last are missing
+    const uint16_t* g = reinterpret_cast<const uint16_t*>(ch.g8) + (size_t)l0 * N + (nh > 0 ? i0 : 0);
+    uint32_t nx[2];
+    auto fetch = [&](int l) {
+      nx[0] = nh > 0 ? __ldg(g + (size_t)l * N) : 0xFFFFu;
+      nx[1] = nh > 1 ? __ldg(g + (size_t)l * N + 1) : 0xFFFFu;
+    };
+    fetch(0);
     for (int l = 0; l < nl; l++) {
-      int a[4];
-#pragma unroll
-      for (int r = 0; r < 4; r++) {
-        a[r] = nx[r];
-        nx[r] = (r >> 1) < nh && l + 1 < nl ? g[r][l + 1] : kG8Missing;
-      }
+      const uint32_t a[4] = {nx[0] & 0xFFu, nx[0] >> 8, nx[1] & 0xFFu, nx[1] >> 8};
+      if (l + 1 < nl) fetch(l + 1);
       U4 w{0, 0, 0, 0};
       if (MODE == kZNormal)
         w = philox_s((uint32_t)(l0 + l), (uint32_t)pair, (uint32_t)rep, (uint32_t)kSZ, key);
+      const float* Pl = sP + l * A * KS;
+      double prod = 1.0;
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const bool m0 = a[2 * h] == kG8Missing, m1 = a[2 * h + 1] == kG8Missing;
-        const float* P0 = sP + l * KT * A + (m0 ? 0 : a[2 * h]);
-        const float* P1 = sP + l * KT * A + (m1 ? 0 : a[2 * h + 1]);
+        const int a0 = m0 ? 0 : (int)a[2 * h], a1 = m1 ? 0 : (int)a[2 * h + 1];
+        const float* P0 = Pl + a0 * KS;
+        const float* P1 = Pl + a1 * KS;
         float2 C[KT];
 #pragma unroll
         for (int k = 0; k < KT; k++) {
-          const float2 X = make_float2(P0[k * A], P1[k * A]);
+          const float2 X = make_float2(P0[k], P1[k]);
           const float2 qq = make_float2(q[h][k], q[h][k]);
           C[k] = k == 0 ? mul2_rn(qq, X) : fma2_rn(qq, X, C[k > 0 ? k - 1 : 0]);
         }
         const float2 T = C[KT - 1];
         if (want_like) {
-          if (!m0) lp.mul(fmax((double)T.x, 1e-50));
-          if (!m1) lp.mul(fmax((double)T.y, 1e-50));
+          // CalcLike's clamp at 1e-50 lies below the least FP32 number, so only a
+          // zero meets it
+          const double x = m0 ? 1.0 : T.x > 0.0f ? (double)T.x : 1e-50;
+          const double y = m1 ? 1.0 : T.y > 0.0f ? (double)T.y : 1e-50;
+          prod *= x * y;
         }
         if (MODE == kZNormal) {
           // z = #{k : C_k < RN(u T)}: the signs of C_k - r (st_zpass_fast.cuh)
@@ -188,14 +206,10 @@ __global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
             t1 = __funnelshift_l(__float_as_uint(D.y), t1, 1);
           }
           const int z0 = __popc(t0), z1 = __popc(t1), one = h ? 65536 : 1;
-          if (!m0) {
-            atomicAdd(&sM[z0 * kUT + threadIdx.x], one);
-            if (ncnt[h]) atomicAdd(&sN[(l * K + z0) * A + a[2 * h]], 1);
-          }
-          if (!m1) {
-            atomicAdd(&sM[z1 * kUT + threadIdx.x], one);
-            if (ncnt[h]) atomicAdd(&sN[(l * K + z1) * A + a[2 * h + 1]], 1);
-          }
+          atomicAdd(&myM[z0 * kUT], m0 ? 0 : one);
+          atomicAdd(&myM[z1 * kUT], m1 ? 0 : one);
+          atomicAdd(&sN[!m0 && ncnt[h] ? l * KA + z0 * A + a0 : spare], 1);
+          atomicAdd(&sN[!m1 && ncnt[h] ? l * KA + z1 * A + a1 : spare], 1);
           if (store_z && h < nh) {
             uint8_t* Z = ch.Z + (size_t)(i0 + h) * 2 * L + l0 + l;
             Z[0] = m0 ? kZMissing : (uint8_t)z0;
@@ -203,6 +217,7 @@ __global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
           }
         }
       }
+      if (want_like) lp.mul(prod);   // four factors of at least 1e-50 at a time
     }
     if (want_like) {
       lp.flush();
@@ -215,12 +230,20 @@ __global__ void __launch_bounds__(kUT) u8_kernel(ChainDev* __restrict__ chains,
         const int v = sN[l * K * A + ka];
         if (v) atomicAdd(&ch.npart[(size_t)ka * L + l0 + l], v);
       }
-      const int r0 = pb * 2 * kUT, nr = min(2 * kUT, N - r0);
+      // ancestry counts, coalesced: element e = (row, k) in steps of kUT
+      const int r0 = pb * 2 * kUT, ne = min(2 * kUT, N - r0) * K;
       int* dst = ch.mpart + (size_t)r0 * K;
-      for (int idx = threadIdx.x; idx < nr * K; idx += kUT) {
-        const int ii = idx / K, k = idx - ii * K;
-        const int v = (sM[k * kUT + (ii >> 1)] >> (16 * (ii & 1))) & 0xFFFF;
-        if (v) atomicAdd(&dst[idx], v);
+      const int dr = kUT / K, dk = kUT - dr * K;
+      int row = threadIdx.x / K, k = threadIdx.x - row * K;
+      for (int e = threadIdx.x; e < ne; e += kUT) {
+        const int v = (sM[k * kUT + (row >> 1)] >> (16 * (row & 1))) & 0xFFFF;
+        if (v) atomicAdd(&dst[e], v);
+        row += dr;
+        k += dk;
+        if (k >= K) {
+          k -= K;
+          row++;
+        }
       }
     }
   }
@@ -271,13 +294,14 @@ size_t u8_smem(const ChainDev& c, int mode) {
   return (size_t)u8_layout(u8_kclass(c.K), c.K, c.A, c.u8_lc, mode).total;
 }
 
-// Loci per chunk: about two CTAs per SM from one chain (a small chain gets one locus
+// Loci per chunk: about one CTA per SM from one chain (a small chain gets one locus
 // per CTA, a large one up to 16 so that a CTA's staging and reductions are shared by
-// more copies), within the shared memory and the room for the partials.  It depends
-// on the chain's shape alone, so ln P(D) is the same in a batch.
+// more copies: 8 chains of N=1000, L=300, K=6 take 37 us with 9 loci, 43 with 5; one
+// such chain 17.8 against 16.9), within the shared memory and the room for the
+// partials.  It depends on the chain's shape alone, so ln P(D) is the same in a batch.
 int u8_plan(int N, int L, int K, int A, long cap) {
   const long blocks = (N + 2 * kUT - 1) / (2 * kUT);
-  long lc = (L * blocks + 148 * 2 - 1) / (148 * 2);
+  long lc = (L * blocks + 148 - 1) / 148;
   if (lc > kUMaxLc) lc = kUMaxLc;
   const int KT = u8_kclass(K);
   while (lc > 1 && (u8_layout(KT, K, A, (int)lc, kZNormal).total > (int)kUSmem ||
