@@ -253,6 +253,7 @@ LaunchSet single(st_chain* c, int ctas) {
   ls.nchains = 1;
   ls.total_ctas = ctas;
   ls.stream = c->ctx->stream;
+  ls.behind = true;
   return ls;
 }
 

@@ -464,6 +464,16 @@ __device__ __forceinline__ bool last_cta_arrive(unsigned* ctr, unsigned total) {
   return last;
 }
 
+// Waits for the kernel before this one on the stream (launch_behind): its writes are
+// visible from here on.
+__device__ __forceinline__ void after_previous_kernel() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// The kernel behind this one may launch from here on, once all blocks have come here.
+__device__ __forceinline__ void next_kernel_may_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // Binary search of the owning chain for a flat tile index.
 __device__ __forceinline__ int find_chain(const int* prefix, int nchains, int t) {
   int lo = 0, hi = nchains - 1;

@@ -199,7 +199,7 @@ int run(int device, const uint32_t* g2, int wpr, int N, int L, int K, const floa
   ls.prefix = dhead->prefix;
   ls.nchains = 1;
   ls.total_ctas = (int)ntiles;
-  ls.stream = stream;
+  ls.stream = stream;   // not ls.behind: the kernel before this one writes the descriptor
   if (launch_zcount(ls, KT, kZNormal, like_out ? kZfLikeAlways : 0, zcount_smem(KT, t.T)) != cudaSuccess)
     return ST_ERR_CUDA;
 

@@ -43,6 +43,7 @@ __device__ __forceinline__ void warp_slot_sums(double v, int G, double* s, int n
 // ---------------------------------------------------------------------------
 constexpr int kStageKA = 16;   // populations x alleles staged per locus (P stage)
 
+template <bool BEHIND>
 __global__ void __launch_bounds__(256, 4)
 locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains,
              int stages) {
@@ -69,10 +70,11 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
   int J = 1;
   while (J * 2 * K <= tpl && J * 2 <= 32) J *= 2;
   const int kslots = tpl / J, j = sub % J, k0 = sub / J;
-  const int rep = *ch.rep;
   const uint32_t key = ch.key;
-  const bool collect = (stages & kLocCollect) && (rep + 1 > ch.burnin);
   const int na = (l < L) ? ch.numalleles[l] : 0;
+  if (BEHIND) after_previous_kernel();
+  const int rep = *ch.rep;
+  const bool collect = (stages & kLocCollect) && (rep + 1 > ch.burnin);
   const bool fstage = (stages & kLocFst) && ch.freqscorr;
   const int numfst = ch.onefst ? 1 : K;
   if (ch.freqscorr && (stages & (kLocP | kLocEps | kLocFst))) {
@@ -275,6 +277,7 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
         ch.SumEps[(size_t)l * A + a] += ch.eps[(size_t)l * A + a];
   }
 
+  if (BEHIND) next_kernel_may_launch();
   // ---- F ------------------------------------------------------------------
   if (fstage) {
     // per-warp sums of each proposal's locus terms, then CTA sums in warp order
@@ -427,8 +430,8 @@ int locus_lanes(int L, int K, int A, long others) {
 }
 
 cudaError_t launch_locus(const LaunchSet& ls, int stages, int block) {
-  locus_kernel<<<ls.total_ctas, block, 0, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, stages);
-  return cudaGetLastError();
+  return launch_behind(ls, locus_kernel<false>, locus_kernel<true>, block, 0, ls.chains, ls.prefix,
+                       ls.nchains, stages);
 }
 
 // ---------------------------------------------------------------------------
@@ -523,6 +526,7 @@ cudaError_t launch_lambda(const LaunchSet& ls, int block) {
 // ---------------------------------------------------------------------------
 // Individual kernel
 // ---------------------------------------------------------------------------
+template <bool BEHIND>
 __global__ void __launch_bounds__(256)
 ind_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains,
            int mode, int stages) {
@@ -540,8 +544,9 @@ ind_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nc
   const int i = tile * gpb + gid;
   const bool ivalid = i < N;
   const bool kvalid = ivalid && k < K;
-  const int rep = *ch.rep;
   const uint32_t key = ch.key;
+  if (BEHIND) after_previous_kernel();
+  const int rep = *ch.rep;
   const bool collect = (stages & kIndCollect) && (rep + 1 > ch.burnin);
   const size_t qi = (size_t)(ivalid ? i : 0) * K + (k < K ? k : 0);
   // USEPOPINFO: flagged individuals keep the migrant-model Q drawn before this
@@ -618,6 +623,7 @@ ind_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nc
     }
   }
 
+  if (BEHIND) next_kernel_may_launch();
   if ((stages & kIndAlpha) && ch.inferalpha && mode != kIndPropose) {
     const int nslot = K + 1;
     const int nwarps = blockDim.x >> 5;
@@ -740,8 +746,8 @@ int ctas_ind(const ChainDev& c, int block) {
 }
 
 cudaError_t launch_ind(const LaunchSet& ls, int mode, int stages, int block) {
-  ind_kernel<<<ls.total_ctas, block, 0, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, mode, stages);
-  return cudaGetLastError();
+  return launch_behind(ls, ind_kernel<false>, ind_kernel<true>, block, 0, ls.chains, ls.prefix,
+                       ls.nchains, mode, stages);
 }
 
 // ---------------------------------------------------------------------------

@@ -332,7 +332,7 @@ __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const P
   }
 }
 
-template <int KT, bool DRAW>
+template <int KT, bool DRAW, bool BEHIND>
 __global__ void __launch_bounds__(kNT, zc_ctas(KT))
 zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains, int flags) {
   extern __shared__ __align__(16) unsigned char smem[];
@@ -354,6 +354,7 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
   const int nT = min(N, i0 + T) - i0;
   const int nT16 = (nT + 15) & ~15;  // whole words; padding genotypes are "missing"
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (BEHIND) after_previous_kernel();
   const int rep = *ch.rep;
   const bool collect = rep + 1 > ch.burnin;
   const bool want_like =
@@ -451,6 +452,7 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
     }
     __syncwarp();
   }
+  if (BEHIND) next_kernel_may_launch();
   __syncthreads();
   if constexpr (DRAW) {
     // thread = row: n_k = cum_{k-1} - cum_k, cum_{-1} = copies present
@@ -485,14 +487,19 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
 
 template <int KT>
 cudaError_t launch_zcount_k(const LaunchSet& ls, int mode, int flags, size_t smem) {
-  auto fn = mode == kZLike ? zcount_kernel<KT, false> : zcount_kernel<KT, true>;
+  auto fn = mode == kZLike ? zcount_kernel<KT, false, false>
+            : ls.behind    ? zcount_kernel<KT, true, true>
+                           : zcount_kernel<KT, true, false>;
   if (smem > 40 * 1024) {   // above the default 48 KB with the static shared memory
     const cudaError_t e =
         cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  fn<<<ls.total_ctas, kNT, smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);
-  return cudaGetLastError();
+  if (mode == kZLike) {
+    fn<<<ls.total_ctas, kNT, smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);
+    return cudaGetLastError();
+  }
+  return launch_behind(ls, fn, fn, kNT, smem, ls.chains, ls.prefix, ls.nchains, flags);
 }
 
 }  // namespace zcount

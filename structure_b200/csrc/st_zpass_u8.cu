@@ -61,10 +61,9 @@ struct LogProduct {
   }
 };
 
-template <int KT, int MODE>
-__global__ void __launch_bounds__(kUT, KT <= 8 ? 4 : 3) u8_kernel(ChainDev* __restrict__ chains,
-                                                 const int* __restrict__ prefix, int nchains,
-                                                 int flags) {
+template <int KT, int MODE, bool BEHIND>
+__global__ void __launch_bounds__(kUT, KT <= 8 ? 4 : 3)
+u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains, int flags) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ double sred[kUT / 32];
   const int c = find_chain(prefix, nchains, blockIdx.x);
@@ -73,6 +72,7 @@ __global__ void __launch_bounds__(kUT, KT <= 8 ? 4 : 3) u8_kernel(ChainDev* __re
   const int N = ch.N, L = ch.L, K = ch.K, A = ch.A;
   const int pb = tile / ch.u8_chunks, l0 = (tile - pb * ch.u8_chunks) * ch.u8_lc;
   const int nl = min(ch.u8_lc, L - l0);
+  if (BEHIND) after_previous_kernel();
   const int rep = *ch.rep;
   const bool collect = rep + 1 > ch.burnin;
   const bool want_like = MODE == kZLike ||
@@ -223,6 +223,7 @@ __global__ void __launch_bounds__(kUT, KT <= 8 ? 4 : 3) u8_kernel(ChainDev* __re
       lp.flush();
       like_acc = lp.s;
     }
+    if (BEHIND) next_kernel_may_launch();
     if (MODE == kZNormal) {
       __syncthreads();
       for (int idx = threadIdx.x; idx < nl * K * A; idx += kUT) {   // locus fastest
@@ -263,19 +264,18 @@ __global__ void __launch_bounds__(kUT, KT <= 8 ? 4 : 3) u8_kernel(ChainDev* __re
 
 template <int KT>
 cudaError_t launch_kt(const LaunchSet& ls, int mode, int flags, size_t smem) {
-  auto go = [&](auto fn) {
+  auto go = [&](auto fn, auto fnb) {
     if (smem > 40 * 1024) {
       const cudaError_t e =
-          cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+          cudaFuncSetAttribute(ls.behind ? fnb : fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
     }
-    fn<<<ls.total_ctas, kUT, smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);
-    return cudaGetLastError();
+    return launch_behind(ls, fn, fnb, kUT, smem, ls.chains, ls.prefix, ls.nchains, flags);
   };
   switch (mode) {
-    case kZNormal: return go(u8_kernel<KT, kZNormal>);
-    case kZLike: return go(u8_kernel<KT, kZLike>);
-    case kZMetro: return go(u8_kernel<KT, kZMetro>);
+    case kZNormal: return go(u8_kernel<KT, kZNormal, false>, u8_kernel<KT, kZNormal, true>);
+    case kZLike: return go(u8_kernel<KT, kZLike, false>, u8_kernel<KT, kZLike, true>);
+    case kZMetro: return go(u8_kernel<KT, kZMetro, false>, u8_kernel<KT, kZMetro, true>);
   }
   return cudaErrorInvalidValue;
 }
