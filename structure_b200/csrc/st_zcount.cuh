@@ -42,7 +42,8 @@ constexpr int kRedStride = 36;     // words per row of the reduction buffer (16-
 // 3 classes 102.5; 2 CTAs 113, 4 CTAs 108), K=8 143 (2 registers 147, two parts
 // 150, 2 CTAs 152), K=10 179 (4 registers 180, 3 CTAs 181, two parts 183,
 // shared-memory sums 186), K=20 382 (6 registers and 1 CTA 417, 14 registers
-// 391, four parts 392, shared-memory sums 528).  Where the table of every
+// 391, four parts 392, shared-memory sums 528).  (K <= 5 has since lost 1.3 % more: the
+// likelihood product predicated, the loci's sign bytes added a pair of rows at a time.)  Where the table of every
 // population fits three CTAs, registers only add selects; above K=8 they make
 // room for two CTAs.
 __host__ __device__ constexpr int zc_ctas(int kt) { return kt <= 8 ? 3 : kt <= 24 ? 2 : 1; }
@@ -174,6 +175,7 @@ __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const P
 #pragma unroll
         for (int j = 0; j < kJN; j += 2) {
           U4 r4;
+          uint32_t s_even[NW > 0 ? NW : 1];
           if (NT > 0) r4 = prun.block_r0(phw ^ (uint32_t)(j >> 1));
 #pragma unroll
           for (int h = 0; h < 2; h++) {
@@ -231,7 +233,12 @@ __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const P
                   y = sign_bytes<kLast>(dy + 4 * w);
                 }
                 s[w] = x + y;
-                lo.all[w] += s[w];
+                if (kRedux)
+                  lo.all[w] += s[w];
+                else if (h == 0)   // two genotypes' bytes in one three-operand addition
+                  s_even[w] = s[w];
+                else
+                  lo.all[w] += s_even[w] + s[w];
                 // 0/1 and 1/1: copy 1 carries allele 1; 1/1: copy 0 does too
                 // (missing: x = y = 0).  As asm, the additions stay predicated
                 // ones; otherwise they turn into masks of several operations.
@@ -250,8 +257,14 @@ __device__ __forceinline__ void zcount_words(int nwords, uint32_t pair0, const P
               }
             }
             if (LIKE) {
-              const float pr = miss ? 1.0f : Tp.x * Tp.y;
-              wprod = ((j + h) & 3) == 0 ? pr : wprod * pr;
+              const float pr = Tp.x * Tp.y;
+              if (((j + h) & 3) == 0)
+                wprod = miss ? 1.0f : pr;
+              else if (kRedux)
+                wprod *= miss ? 1.0f : pr;
+              else if (!miss)   // one predicated product; a select of 1 above K=5, where
+                                // it measured the same or better
+                asm volatile("mul.rn.f32 %0, %0, %1;" : "+f"(wprod) : "f"(pr));
               if (((j + h) & 3) == 3) {
                 wmin = fminf(wmin, wprod);
                 wlike += __logf(wprod);
