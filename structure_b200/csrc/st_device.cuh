@@ -61,7 +61,6 @@ __device__ __forceinline__ U4 philox_s(uint32_t a, uint32_t b, uint32_t rep,
 struct PhiloxRun {
   uint32_t head;         // hi(M1 rep) ^ k0_0 ^ (stream << 24)
   uint32_t y1, z0, z2, w3;
-  __device__ __forceinline__ PhiloxRun() {}
   __device__ __forceinline__ PhiloxRun(uint32_t a, uint32_t rep, uint32_t stream,
                                        uint32_t seed32) {
     const uint64_t p0 = (uint64_t)0xD2511F53u * a, p1 = (uint64_t)0xCD9E8D57u * rep;

@@ -4,19 +4,18 @@
 // (Updates/UpdateP.c:60-99 GetNumFromPops) and ancestry counts m[i][k]
 // (Updates/UpdateQ.c:17-35 GetNumLociPop) for the next sweep's P and Q
 // updates, and, when asked, reduces ln P(D|Q,P) (CalcLike.c:75-133,387-426).
-// The same tiling serves the Metropolis Q move's likelihood ratio
-// (CalcLike.c:281-345) and the initial random Z (Init.c:125-169).
+// The Metropolis Q move's likelihood ratio (CalcLike.c:281-345) and the initial random
+// Z (Init.c:125-169) are passes over the same data.
 //
-// Fast path (biallelic, 2 bits per genotype, locus-major rows):
-//   CTA = W warps; lane = one locus; each warp walks the T individuals of its
-//   chunk, 16 genotypes per 32-bit word.  P[l][k][0..1] lives in registers,
-//   Q rows of the chunk in shared memory (broadcast reads).  n[l][k][a] is a
-//   lane-private shared-memory histogram (lane-minor, conflict-free); m[i][k]
-//   is reduced across the warp's 32 loci with one redux.sync per step on
-//   7-bit packed fields.  Counts are added into one histogram per chain,
-//   n[k][a][l] and m[i][k], with integer reductions (cleared by the host
-//   before the pass); the Metropolis log ratios leave as per-CTA partials
-//   ldpart[group][i].
+// This file holds the dispatchers, the tile rules, the generic path (FP64 arithmetic,
+// injected uniforms, stored Z on one-byte data) and the packing of one-byte data.  The
+// paths by data and chain:
+//   2 bits per genotype   draws and counts, ln P(D)    st_zcount.cuh
+//                         Metropolis ratio             st_zmetro.cuh
+//                         Init, recount; Z stored,     st_zpass_fast.cuh
+//                         PFROMPOPFLAGONLY
+//   one byte per copy     draws, ln P(D), Metropolis   st_zpass_u8.cu
+//                         the rest                     zpass_u8_kernel, below
 #include <cmath>
 #include <cstdio>
 #include "st_device.cuh"
@@ -25,8 +24,6 @@
 namespace st {
 
 namespace {
-
-constexpr float kLikeTinyF = 1e-30f;
 
 // Deterministic block sum of one double per thread (fixed tree order).
 __device__ __forceinline__ double block_sum_d(double v, double* sred) {

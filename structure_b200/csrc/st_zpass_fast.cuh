@@ -1,4 +1,7 @@
-// st_zpass_fast.cuh -- the biallelic fast path of the data pass (templates).
+// st_zpass_fast.cuh -- the general pass over biallelic 2-bit data (templates): the
+// initial random Z, counts of a given Z, and the draws and ln P(D) of chains that store
+// Z or use PFROMPOPFLAGONLY.  The counting pass of every other chain is st_zcount.cuh,
+// the Metropolis pass st_zmetro.cuh.
 // Instantiated per K class in st_zpass_k*.cu so the classes compile in
 // parallel; st_zpass.cu holds the dispatcher and the generic path.
 //
@@ -20,7 +23,6 @@ namespace st {
 namespace zfast {
 
 
-constexpr float kLikeTinyF = 1e-30f;
 // ln P(D) fast path: the genotype terms Q.P(copy 0) * Q.P(copy 1) of four
 // genotypes are multiplied in FP32 and logged once.  A product of four above
 // this bound has every factor above it too (factors are <= 1), so no partial
@@ -94,6 +96,8 @@ __host__ __device__ inline ZLayout zlayout(int KT, int K, int T, int nw32, int m
   ZLayout z;
   size_t o = 0;
   z.q2 = o; if (useP) o = zalign16(o + (size_t)T * KT2 * 8);            // (q,q) pairs
+  // kZMetro: no pass of this file, but its size takes part in the choice of the tile,
+  // on which the grouping of the Metropolis log ratios' sums depends
   z.t2 = o; if (mode == kZMetro) o = zalign16(o + (size_t)T * KT2 * 8);  // (t,t) pairs
   z.x = o;  if (useP) o = zalign16(o + (size_t)(zsingles(KT) ? 1 : 3) * KT * nw32 * 8);
   z.ld = o; if (mode == kZMetro) o = zalign16(o + (size_t)T * (nw32 / 32) * 4);   // per warp
