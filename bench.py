@@ -199,7 +199,7 @@ def load_peaks():
 def read_profile_figure(key):
     """A figure of the committed ncu summary of the Z pass (a line "key: value"),
     if any."""
-    path = os.path.join(ROOT, "profiles", "zpass_b2g_snp2000x50000_k5_batch20.txt")
+    path = os.path.join(ROOT, "profiles", "zcount_snp2000x50000_k5_batch20.txt")
     try:
         with open(path) as f:
             for line in f:
@@ -366,7 +366,7 @@ def run_ours(args):
     alu_peak = 148 * 128 * sm_mhz * 1e6 / 1e12
     # issue roofline of the same kernel, the limit it actually meets: warp
     # instructions per 32 genotypes from the ncu capture of a collecting launch
-    # (profiles/zpass_b2g_snp2000x50000_k5_batch20.txt), as the timed launches are
+    # (profiles/zcount_snp2000x50000_k5_batch20.txt), as the timed launches are
     inst_per_32 = read_profile_figure("inst_per_32_genotypes")
     issue_achieved = (B * N * L / 32 * inst_per_32 / (zavg / 1e3) / 1e12) if inst_per_32 else None
     issue_peak = 148 * 4 * sm_mhz * 1e6 / 1e12
@@ -404,7 +404,7 @@ def run_ours(args):
         "roofline": {"bound": "hbm", "achieved": round(achieved, 2), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 5), "traffic": traffic,
                      "peak_source": peak_kind,
-                     "kernel": f"zpass_b2g_kernel<K class {api.fast_class(K)}, Normal, 8 warps> "
+                     "kernel": f"zcount_kernel<K class {api.fast_class(K)}> "
                                f"(batched, {B} chains)",
                      "avg_launch_ms": round(zavg, 4),
                      "algorithmic_bytes_per_launch": int(alg_bytes)},
@@ -575,7 +575,7 @@ def _alu_roofline(copies_by_kclass, zpass_ms, sm_mhz):
     ach = ops / (zpass_ms / 1e3) / 1e12
     peak = 148 * 128 * sm_mhz * 1e6 / 1e12
     return {"bound": "alu", "achieved": round(ach, 3), "peak": round(peak, 2), "unit": "Top/s",
-            "frac": round(ach / peak, 4), "kernel": "zpass_b2g_kernel (per K class)",
+            "frac": round(ach / peak, 4), "kernel": "zcount_kernel (per K class)",
             "avg_zpass_ms_per_sweep": round(zpass_ms, 4),
             "note": "(2K+2) FP32 + ~10 int (Philox/4) + 0.5 log per allele copy at the K "
                     "class; peak = 148 SM x 128 lanes x median SM clock; Z-pass time from "
