@@ -66,9 +66,9 @@ enum : int {
 };
 
 // Locus-kernel stages.
-// kLocClear: the P stage zeroes the allele counts that it has read, and kIndClear
-// (with the last launch of a sweep's Q update) the ancestry counts, so that the
-// sweep's Z pass needs no memsets (kZfCleared).
+// kLocClear: the P stage zeroes every allele count once it has read those it needs, and
+// kIndClear (with the last launch of a sweep's Q update) the ancestry counts, so that
+// the sweep's Z pass needs no memsets (kZfCleared).
 enum : int { kLocP = 0x1, kLocEps = 0x2, kLocFst = 0x4, kLocCollect = 0x8, kLocClear = 0x10 };
 // Individual-kernel modes and stages.
 enum : int { kIndGibbs = 0, kIndPropose = 1, kIndAccept = 2, kIndNone = 3 };

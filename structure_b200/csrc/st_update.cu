@@ -34,6 +34,15 @@ __device__ __forceinline__ void warp_slot_sums(double v, int G, double* s, int n
   if (lane < G && slot >= 0 && slot < nslot) s[warp * nslot + slot] = v;
 }
 
+// Zeroes the allele counts of population k at locus l, alleles a0, a0 + step, ... of
+// all A: packed genotypes and counts that a caller sets may hold alleles at or above
+// the locus' own number, which the P stage does not read.
+__device__ __forceinline__ void clear_counts(const ChainDev& ch, int k, int l, int a0, int step) {
+  for (int cc = 0; cc < ch.cnt_chunks; cc++)
+    for (int a = a0; a < ch.A; a += step)
+      ch.npart[(((size_t)cc * ch.K + k) * ch.A + a) * ch.L + l] = 0;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -103,11 +112,8 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       if (kv) {
         for (int a = j; a < na && a < kMaxAlleles; a += J) {
           int n = 0;
-          for (int cc = 0; cc < ch.cnt_chunks; cc++) {
-            int32_t* cnt = &ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
-            n += *cnt;
-            if (stages & kLocClear) *cnt = 0;
-          }
+          for (int cc = 0; cc < ch.cnt_chunks; cc++)
+            n += ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
           const double shape = ch.freqscorr ? ch.eps[(size_t)l * A + a] * sFrac[k] + (double)n
                                             : ch.lambda[k] + (double)n;
           lg[nmine] = (double)log_gamma_draw_f32((float)shape, (uint32_t)(base + a),
@@ -116,6 +122,7 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
           nmine++;
         }
       }
+      if ((stages & kLocClear) && l < L && k < K) clear_counts(ch, k, l, j, J);
       M = group_max(M, J);
       double S = 0.0;
       for (int t = 0; t < nmine; t++) S += exp(lg[t] - M);
@@ -150,11 +157,8 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       const size_t base = ((size_t)l * K + k) * A;
       auto shape_of = [&](int a) {
         int n = 0;
-        for (int cc = 0; cc < ch.cnt_chunks; cc++) {
-          int32_t* cnt = &ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
-          n += *cnt;
-          if (stages & kLocClear) *cnt = 0;
-        }
+        for (int cc = 0; cc < ch.cnt_chunks; cc++)
+          n += ch.npart[(((size_t)cc * K + k) * A + a) * L + l];
         // eps (1-F)/F + n (Updates/UpdateP.c:161-164), with (1-F)/F formed once per CTA
         if (ch.freqscorr) return ch.eps[(size_t)l * A + a] * sFrac[k] + (double)n;
         return ch.lambda[k] + (double)n;
@@ -209,6 +213,9 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       }
     }
   }
+
+  if ((stages & kLocClear) && tpl == 1 && lvalid)
+    for (int k = 0; k < K; k++) clear_counts(ch, k, l, 0, 1);
 
   if (pstage) {
     // rows l0 .. l0 + nl - 1 of P, log P and PSum are contiguous: [l][k][a]
