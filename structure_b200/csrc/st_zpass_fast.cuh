@@ -199,6 +199,9 @@ __device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, in
   const int lane = za.lane, my_word = za.my_word, my_shift = za.my_shift;
   [[maybe_unused]] const int moff = lane < K ? lane : lane - K + KT;
   [[maybe_unused]] const bool second = lane >= K;
+  // the signs of the K - 1 thresholds without those of the class' padding, which count
+  // where a weight is negative (a caller may set any Q and P): z stays below K
+  [[maybe_unused]] const uint32_t zkeep = 0xFFFFFFFFu << (KT - K);
   const uint32_t prep = za.prep, key = za.key, stream = za.stream;
   const bool valid = za.valid, pfonly = EXT && za.pfonly, store_z = EXT && za.store_z;
     // Philox blocks of this lane's locus and sweep: b = individual pair.  i0 is
@@ -277,6 +280,10 @@ __device__ __forceinline__ void zword_loop(const ZArgs& za, double& like_acc, in
                 const float2 D = add2_rn(Cs[k], NR);
                 t0 = __funnelshift_l(__float_as_uint(D.x), t0, 1);
                 t1 = __funnelshift_l(__float_as_uint(D.y), t1, 1);
+              }
+              if (KT > 12) {   // classes wider than K: see zkeep
+                t0 &= zkeep;
+                t1 &= zkeep;
               }
               z0 = __popc(t0);
               z1 = __popc(t1);

@@ -153,6 +153,9 @@ u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nch
     }
     const bool store_z = MODE == kZNormal && (flags & kZfStoreZ) && ch.Z;
     const int spare = nl * K * A, KA = K * A;
+    // the signs of the K - 1 thresholds: those of the class' padding count only where
+    // a weight is negative (a caller may set any Q and P), and z then stays below K
+    const uint32_t zkeep = 0xFFFFFFFFu << (KT - K);
     int* myM = sM + threadIdx.x;
     LogProduct lp;
     // the pair's copies at a locus: two 16-bit loads side by side; individuals beyond
@@ -205,7 +208,7 @@ u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nch
             t0 = __funnelshift_l(__float_as_uint(D.x), t0, 1);
             t1 = __funnelshift_l(__float_as_uint(D.y), t1, 1);
           }
-          const int z0 = __popc(t0), z1 = __popc(t1), one = h ? 65536 : 1;
+          const int z0 = __popc(t0 & zkeep), z1 = __popc(t1 & zkeep), one = h ? 65536 : 1;
           atomicAdd(&myM[z0 * kUT], m0 ? 0 : one);
           atomicAdd(&myM[z1 * kUT], m1 ? 0 : one);
           atomicAdd(&sN[!m0 && ncnt[h] ? l * KA + z0 * A + a0 : spare], 1);
