@@ -1664,8 +1664,9 @@ static int batch_layout(st_batch* b, bool keep_groups) {
   for (int j = 0; j < n; j++) {
     st_chain* c = b->chains[j];
     b->table[j] = c->h;
-    // with two alleles the lanes per locus change no bit of P (a sum of two terms),
-    // so a batch takes fewer of them; with more, every chain keeps its own
+    // with two alleles the lanes per locus change no bit of P (a sum of two terms) nor
+    // of the eps and F sums (their order does not follow the lanes), so a batch takes
+    // fewer of them; with more, every chain keeps its own
     if (c->h.A <= 2)
       b->table[j].loc_tpl = locus_lanes(c->h.L, c->h.K, c->h.A, total_loci - c->h.L);
     if (!b->fast && b->u8) {

@@ -43,6 +43,43 @@ __device__ __forceinline__ void clear_counts(const ChainDev& ch, int k, int l, i
       ch.npart[(((size_t)cc * ch.K + k) * ch.A + a) * ch.L + l] = 0;
 }
 
+// sum + the first n slots' values in order; a locus' tpl lanes hold kslots slots of
+// tpl / kslots lanes each, and a slot's first lane its value.
+__device__ __forceinline__ double add_slots(double sum, double v, int kslots, int n, int tpl) {
+  if (kslots == 1) return sum + v;
+  for (int q = 0; q < n; q++) sum += __shfl_sync(0xffffffffu, v, q * (tpl / kslots), tpl);
+  return sum;
+}
+
+// Sum of p[0], p[stride], ... (n values) by one warp as a balanced binary tree over
+// aligned pairs: zeros beyond n, so two partitions of the same items into 2^a and 2^b
+// items per value, summed within a value by the same tree, give the same bits.  A lane
+// takes an aligned run of 2^c values, four loads at a time.
+__device__ __forceinline__ double warp_tree_sum(const double* p, size_t stride, int n) {
+  int run = 1;
+  while (32 * run < n) run *= 2;
+  const int b0 = (int)(threadIdx.x & 31) * run;
+  auto at = [&](int b) { return b < n ? p[(size_t)b * stride] : 0.0; };
+  double v;
+  if (run == 1) {
+    v = at(b0);
+  } else if (run == 2) {
+    v = at(b0) + at(b0 + 1);
+  } else {
+    double done[28];   // done[i]: a finished tree of 4 * 2^i values
+    v = 0.0;
+    for (int g = 0; g < run / 4; g++) {
+      const int b = b0 + 4 * g;
+      v = (at(b) + at(b + 1)) + (at(b + 2) + at(b + 3));
+      int i = 0;
+      for (int m = g; m & 1; m >>= 1) v = done[i++] + v;
+      done[i] = v;
+    }
+  }
+  for (int off = 1; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+  return v;
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -256,19 +293,22 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
       e2 = ch.eps[(size_t)l * A + a2];
       open = (e1 + d < 1.0) && (e2 - d > 0.0);
     }
-    if (open && j == 0) {
-      for (int k = k0; k < K; k += kslots) {
+    // the populations' terms are added in their order, whatever the lanes, so that a
+    // chain's sums are the same bits at every number of lanes (batch_layout)
+    for (int kb = 0; kb < K; kb += kslots) {
+      const int k = kb + k0;
+      double s = 0.0;
+      if (open && j == 0 && k < K) {
         const double frac = sFrac[k];
         const size_t base = ((size_t)l * K + k) * A;
         const double lp1 = (double)ch.logP[base + a1];
         const double lp2 = (double)ch.logP[base + a2];
-        double s = lgamma_2m2(frac * e1, frac * e2, frac * (e1 + d), frac * (e2 - d));
+        s = lgamma_2m2(frac * e1, frac * e2, frac * (e1 + d), frac * (e2 - d));
         s += frac * d * lp1;
         s -= frac * d * lp2;
-        sum += s;
       }
+      sum = add_slots(sum, s, kslots, min(kslots, K - kb), tpl);
     }
-    sum = group_sum(sum, tpl);
     if (open && sub == 0) {
       const double lam = ch.lambda[0];
       if (lam != 1.0) sum += log(pow((e1 + d) * (e2 - d) / e1 / e2, lam - 1.0));
@@ -287,18 +327,22 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
   if (BEHIND) next_kernel_may_launch();
   // ---- F ------------------------------------------------------------------
   if (fstage) {
-    // per-warp sums of each proposal's locus terms, then CTA sums in warp order
+    // Each proposal's locus terms are summed as one balanced tree over the loci: within
+    // a warp, over the CTA's warps and over the CTAs, so that the sum is the same bits
+    // at every number of lanes per locus.
     const int nwarps = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // population k's terms over this lane's alleles j, j + J, ..., in pairs
+    // population k's terms over this lane's alleles j, j + J, ..., in pairs; with two
+    // alleles the first lane takes the pair (its lanes depend on the launch)
+    const int js = A <= 2 ? 1 : J;
     auto fterm = [&](int k, double nf) {
       double v = 0.0;
-      if (l < L && k < K && nf > 0.0 && nf < 1.0) {
+      if (l < L && k < K && j < js && nf > 0.0 && nf < 1.0) {
         const double nfr = (1.0 - nf) / nf, ofr = sFrac[k];
         const size_t base = ((size_t)l * K + k) * A;
         int a = j;
-        for (; a + J < na; a += 2 * J) {
-          const double e0 = ch.eps[(size_t)l * A + a], e1 = ch.eps[(size_t)l * A + a + J];
-          const double lp0 = (double)ch.logP[base + a], lp1 = (double)ch.logP[base + a + J];
+        for (; a + js < na; a += 2 * js) {
+          const double e0 = ch.eps[(size_t)l * A + a], e1 = ch.eps[(size_t)l * A + a + js];
+          const double lp0 = (double)ch.logP[base + a], lp1 = (double)ch.logP[base + a + js];
           v += (nfr - ofr) * e0 * lp0 + (nfr - ofr) * e1 * lp1 -
                lgamma_2m2(nfr * e0, nfr * e1, ofr * e0, ofr * e1);
         }
@@ -314,33 +358,31 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
     for (int kb = 0; kb < K; kb += kslots) {
       const int k = kb + k0;
       double v = fterm(k, sNF[ch.onefst || k >= K ? 0 : k]);
-      if (ch.onefst) {
-        vone += v;
-      } else {   // over the allele slots and the warp's loci
-        for (int off = 1; off < J; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      for (int off = 1; off < J; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+      if (ch.onefst) {   // the populations in their order
+        vone = add_slots(vone, v, kslots, min(kslots, K - kb), tpl);
+      } else {   // over the warp's loci
         for (int off = tpl; off < 32; off <<= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
         if (lane < tpl && j == 0 && k < K) sF[warp * numfst + k] = v;
       }
     }
     if (ch.onefst) {
-      for (int off = 16; off > 0; off >>= 1) vone += __shfl_xor_sync(0xffffffffu, vone, off);
+      for (int off = tpl; off < 32; off <<= 1) vone += __shfl_xor_sync(0xffffffffu, vone, off);
       if (lane == 0) sF[warp] = vone;
     }
     __syncthreads();
     const int nblocks = (L * tpl + blockDim.x - 1) / blockDim.x;
     if (threadIdx.x < numfst) {
-      double s = 0.0;
-      for (int w = 0; w < nwarps; w++) s += sF[w * numfst + threadIdx.x];
-      ch.redpart[(size_t)tile * numfst + threadIdx.x] = s;
+      const double* f = sF + threadIdx.x;   // 8 warps
+      ch.redpart[(size_t)tile * numfst + threadIdx.x] =
+          ((f[0] + f[numfst]) + (f[2 * numfst] + f[3 * numfst])) +
+          ((f[4 * numfst] + f[5 * numfst]) + (f[6 * numfst] + f[7 * numfst]));
     }
     if (last_cta_arrive(&ch.ctr[kCtrLocus], (unsigned)nblocks)) {
       // a warp per proposal adds the CTAs' sums (one thread a proposal waited for
       // each load in turn)
       for (int f = warp; f < numfst; f += nwarps) {
-        double s = 0.0;
-#pragma unroll 4
-        for (int b = lane; b < nblocks; b += 32) s += ch.redpart[(size_t)b * numfst + f];
-        for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
+        const double s = warp_tree_sum(ch.redpart + f, numfst, nblocks);
         if (lane == 0) sTot[f] = s;
       }
       __syncthreads();
