@@ -301,7 +301,7 @@ void choose_tile(const st_model* m, int N, int L, int K, int* T, int* W, int* R)
       while (t > 32 && !fits(t, 112 * 1024)) t -= 16;
     }
   }
-  while (t > 16 && zpass_smem_all(KT, K, t, w) > 200 * 1024) t -= 16;
+  while (t > 16 && zpass_smem_all(KT, K, t, w) > kMaxDynamicSmem) t -= 16;
   int r = m->tile_r;
   if (r <= 0) {
     const long lblocks = (L + 32 * w - 1) / (32 * w);
@@ -1768,7 +1768,7 @@ static bool set_tile(st_chain* c, int T, int R) {
   ChainDev& h = c->h;
   if (!c->fast || T < c->tile_min_t || R < c->tile_min_r || (T & 15)) return false;
   const size_t smem = zpass_smem_all(c->KT, h.K, T, h.tileW);
-  if (smem > 200 * 1024) return false;
+  if (smem > kMaxDynamicSmem) return false;
   h.tileT = T;
   h.tileR = R;
   h.nchunks = (h.N + T - 1) / T;

@@ -16,6 +16,19 @@ struct LaunchSet {
   bool behind = false;   // the launch may start while the kernel before it drains
 };
 
+// Dynamic shared memory that the planners of the data passes give a CTA at most.
+constexpr size_t kMaxDynamicSmem = 200 * 1024;
+
+// Lets `fn` be launched with `smem` bytes of dynamic shared memory.  The limit is the
+// function's, for every context and thread on the device, so it is always set to the
+// same ceiling: set to a launch's own size, another thread could lower it between
+// this thread's setting and its launch.
+template <typename F>
+inline cudaError_t allow_dynamic_smem(F* fn, size_t smem) {
+  if (smem <= 40 * 1024) return cudaSuccess;   // the default is 48 KB with the static part
+  return cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem);
+}
+
 // Launches `fn`, or with ls.behind its instantiation `fnb`, which may start while the
 // kernel before it on the stream drains (programmatic dependent launch).  fnb calls
 // st_device.cuh's after_previous_kernel before it touches anything that a sweep's kernels

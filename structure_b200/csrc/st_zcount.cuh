@@ -503,11 +503,7 @@ cudaError_t launch_zcount_k(const LaunchSet& ls, int mode, int flags, size_t sme
   auto fn = mode == kZLike ? zcount_kernel<KT, false, false>
             : ls.behind    ? zcount_kernel<KT, true, true>
                            : zcount_kernel<KT, true, false>;
-  if (smem > 40 * 1024) {   // above the default 48 KB with the static shared memory
-    const cudaError_t e =
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_dynamic_smem(fn, smem)) return e;
   if (mode == kZLike) {
     fn<<<ls.total_ctas, kNT, smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);
     return cudaGetLastError();

@@ -196,11 +196,7 @@ zmetro_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
 template <int KT>
 cudaError_t launch_zmetro_k(const LaunchSet& ls, int flags, size_t smem) {
   auto fn = zmetro_kernel<KT>;
-  if (smem > 40 * 1024) {   // above the default 48 KB
-    const cudaError_t e =
-        cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (const cudaError_t e = allow_dynamic_smem(fn, smem)) return e;
   fn<<<ls.total_ctas, 32 * width(KT), smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);
   return cudaGetLastError();
 }

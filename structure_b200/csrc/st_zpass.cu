@@ -97,7 +97,7 @@ int zc_ctas_of(int kt);
 
 size_t zcount_smem(int KT, int T) { return zcount::zc_layout_total(KT, T); }
 bool zcount_fits(int KT, int T) {
-  return T >= kZcountMinT && T <= kZcountMaxT && T % 16 == 0 && zcount_smem(KT, T) <= 200 * 1024;
+  return T >= kZcountMinT && T <= kZcountMaxT && T % 16 == 0 && zcount_smem(KT, T) <= kMaxDynamicSmem;
 }
 long zcount_ctas(int N, int L, CountTile t) {
   const long blocks = (L + 255) / 256;   // 8 warps of 32 loci

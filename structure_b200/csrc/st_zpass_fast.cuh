@@ -582,8 +582,7 @@ cudaError_t launch_b2g_kw(const LaunchSet& ls, int mode, int flags, size_t smem)
 #define ST_ZCASE(M)                                                                        \
   case M: {                                                                                \
     auto fn = zpass_b2g_kernel<KT, M, W>;                                                   \
-    if (smem > 40 * 1024) /* above the default 48 KB with the static smem */            \
-      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
+    if (const cudaError_t e = allow_dynamic_smem(fn, smem)) return e;                      \
     fn<<<grid, block, smem, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, flags);         \
     return cudaGetLastError();                                                             \
   }

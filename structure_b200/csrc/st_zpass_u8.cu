@@ -268,11 +268,7 @@ u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nch
 template <int KT>
 cudaError_t launch_kt(const LaunchSet& ls, int mode, int flags, size_t smem) {
   auto go = [&](auto fn, auto fnb) {
-    if (smem > 40 * 1024) {
-      const cudaError_t e =
-          cudaFuncSetAttribute(ls.behind ? fnb : fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-      if (e != cudaSuccess) return e;
-    }
+    if (const cudaError_t e = allow_dynamic_smem(ls.behind ? fnb : fn, smem)) return e;
     return launch_behind(ls, fn, fnb, kUT, smem, ls.chains, ls.prefix, ls.nchains, flags);
   };
   switch (mode) {
@@ -311,8 +307,8 @@ int u8_plan(int N, int L, int K, int A, long cap) {
                     u8_layout(KT, K, A, (int)lc, kZMetro).total > (int)kUSmem))
     lc--;
   while (lc <= kUMaxLc && blocks * ((L + lc - 1) / lc) > cap) lc++;
-  if (lc > kUMaxLc || u8_layout(KT, K, A, (int)lc, kZNormal).total > 200 * 1024 ||
-      u8_layout(KT, K, A, (int)lc, kZMetro).total > 200 * 1024)
+  if (lc > kUMaxLc || u8_layout(KT, K, A, (int)lc, kZNormal).total > (int)kMaxDynamicSmem ||
+      u8_layout(KT, K, A, (int)lc, kZMetro).total > (int)kMaxDynamicSmem)
     return 0;
   return (int)lc;
 }
