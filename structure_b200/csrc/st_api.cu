@@ -702,17 +702,22 @@ extern "C" int st_data_upload(st_ctx* ctx, const st_data_desc* d, st_data** out)
     rc = ctx_alloc(ctx, n, &p, nullptr, &s->bytes);
     if (rc) { st_data_destroy(s); return rc; }
     s->g8 = (uint8_t*)p;
-    // stage the int32 genotypes through a temporary device buffer in slices
+    // stage the int32 genotypes through a temporary device buffer: whole rows (a copy's
+    // loci) at a time, or pieces of one row that is longer than the buffer
     const size_t slice = (size_t)1 << 26;
+    const int cols = (int)std::min((size_t)L, slice);
+    const int rows = (int)std::min((size_t)2 * N, std::min(slice / cols, (size_t)1 << 20));
     int32_t* tmp = nullptr;
-    rc = cuda_check(ctx, cudaMalloc(&tmp, sizeof(int32_t) * std::min(n, slice)), "staging");
+    rc = cuda_check(ctx, cudaMalloc(&tmp, sizeof(int32_t) * (size_t)rows * cols), "staging");
     if (rc) { st_data_destroy(s); return rc; }
-    for (size_t off = 0; off < n; off += slice) {
-      size_t m = std::min(slice, n - off);
-      cudaMemcpy(tmp, d->geno + off, sizeof(int32_t) * m, cudaMemcpyHostToDevice);
-      launch_pack_u8(tmp, s->g8, off, m, N, L, 0);
-      ctx->launches++;
-    }
+    for (size_t r = 0; r < (size_t)2 * N; r += rows)
+      for (size_t c = 0; c < (size_t)L; c += cols) {
+        const int nr = (int)std::min((size_t)rows, (size_t)2 * N - r);
+        const int nc = (int)std::min((size_t)cols, (size_t)L - c);
+        cudaMemcpy(tmp, d->geno + r * L + c, sizeof(int32_t) * (size_t)nr * nc, cudaMemcpyHostToDevice);
+        launch_pack_u8(tmp, s->g8, r, nr, (int)c, nc, N, 0);
+        ctx->launches++;
+      }
     cudaDeviceSynchronize();
     cudaFree(tmp);
     rc = cuda_check(ctx, cudaGetLastError(), "pack genotypes");

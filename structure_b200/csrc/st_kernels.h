@@ -143,8 +143,8 @@ cudaError_t launch_inj_metro_propose(const ChainDev& h, ChainDev* d_chain, const
                                      int* taken, cudaStream_t s);
 cudaError_t launch_inj_metro_accept(const ChainDev& h, ChainDev* d_chain, const double* uni,
                                     const int* taken, cudaStream_t s);
-cudaError_t launch_pack_u8(const int32_t* geno, uint8_t* g8, size_t off, size_t n, int N, int L,
-                           cudaStream_t s);
+cudaError_t launch_pack_u8(const int32_t* geno, uint8_t* g8, size_t row0, int rows, int col0,
+                           int cols, int N, cudaStream_t s);
 cudaError_t launch_clear_counts(const ChainDev* d_table, int nchains, cudaStream_t s);
 cudaError_t launch_init_chain(const ChainDev& h, ChainDev* d_chain, int* d_prefix,
                               const double* eps0, int arows, float q0, float lq0, double f0,

@@ -246,10 +246,11 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
   ChainDev& ch = chains[c];
   const int tile = blockIdx.x - prefix[c];
   const int N = ch.N, L = ch.L, K = ch.K, A = ch.A;
+  // neighbouring threads are neighbouring individuals, as the genotypes [L][N][2] lie
   const size_t idx = (size_t)tile * blockDim.x + threadIdx.x;
   const bool active = idx < (size_t)N * L;
-  const int i = active ? (int)(idx / L) : 0;
-  const int l = active ? (int)(idx - (size_t)i * L) : 0;
+  const int l = active ? (int)(idx / N) : 0;
+  const int i = active ? (int)(idx - (size_t)l * N) : 0;
   const int rep = *ch.rep;
   const bool collect = rep + 1 > ch.burnin;
   const bool want_like = (mode == kZLike) ||
@@ -342,23 +343,33 @@ cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags) {
   return cudaGetLastError();
 }
 
-// int32 reference genotypes [N][2][L] (-9 missing), elements off .. off + n - 1, to one
-// byte per copy (0xFF missing) in [L][N][2].
-__global__ void pack_u8_kernel(const int32_t* __restrict__ geno, uint8_t* __restrict__ g8, size_t off,
-                               size_t n, int N, int L) {
-  for (size_t j = blockIdx.x * (size_t)blockDim.x + threadIdx.x; j < n;
-       j += (size_t)gridDim.x * blockDim.x) {
-    const int v = geno[j];
-    const size_t row = (off + j) / L, l = off + j - row * L;   // row = 2 i + line
-    g8[l * (size_t)N * 2 + row] = (v < 0 || v > 254) ? kG8Missing : (uint8_t)v;
-  }
+// int32 reference genotypes (-9 missing) of `rows` copies (row = 2 i + line, from row0)
+// at `cols` loci (from col0), [rows][cols], to one byte per copy (0xFF missing) in
+// [L][N][2].  A CTA turns a tile in shared memory: loads run along the loci, stores
+// along the copies.
+constexpr int kPackTile = 64;
+
+__global__ void __launch_bounds__(256)
+pack_u8_kernel(const int32_t* __restrict__ geno, uint8_t* __restrict__ g8, size_t row0, int rows,
+               int col0, int cols, size_t nrows) {
+  __shared__ uint8_t tile[kPackTile][kPackTile + 4];   // [locus][row]; odd in words
+  const int r0 = blockIdx.y * kPackTile, c0 = blockIdx.x * kPackTile;
+  const int x = threadIdx.x % kPackTile, y = threadIdx.x / kPackTile;
+  for (int r = y; r < kPackTile; r += 256 / kPackTile)
+    if (r0 + r < rows && c0 + x < cols) {
+      const int v = geno[(size_t)(r0 + r) * cols + c0 + x];
+      tile[x][r] = (v < 0 || v > 254) ? kG8Missing : (uint8_t)v;
+    }
+  __syncthreads();
+  for (int c = y; c < kPackTile; c += 256 / kPackTile)
+    if (r0 + x < rows && c0 + c < cols)
+      g8[(size_t)(col0 + c0 + c) * nrows + row0 + r0 + x] = tile[c][x];
 }
 
-cudaError_t launch_pack_u8(const int32_t* geno, uint8_t* g8, size_t off, size_t n, int N, int L,
-                           cudaStream_t s) {
-  int blocks = (int)((n + 255) / 256);
-  if (blocks > 148 * 16) blocks = 148 * 16;
-  pack_u8_kernel<<<blocks, 256, 0, s>>>(geno, g8, off, n, N, L);
+cudaError_t launch_pack_u8(const int32_t* geno, uint8_t* g8, size_t row0, int rows, int col0,
+                           int cols, int N, cudaStream_t s) {
+  const dim3 grid((cols + kPackTile - 1) / kPackTile, (rows + kPackTile - 1) / kPackTile);
+  pack_u8_kernel<<<grid, 256, 0, s>>>(geno, g8, row0, rows, col0, cols, (size_t)N * 2);
   return cudaGetLastError();
 }
 
