@@ -53,6 +53,23 @@ def make_data():
 # METROFREQ cycle = 9 Gibbs + 1 Metropolis sweep per ten); time scales
 # linearly in L.
 # ---------------------------------------------------------------------------
+REF_LIB = os.path.join(ROOT, "oracle", "_ref", "libstref.so")
+
+
+def reference_missing():
+    """Why the reference's CPU functions cannot be timed here, or None."""
+    if os.path.exists(REF_LIB):
+        return None
+    from oracle import oracle
+    if not os.path.isdir(oracle.REF_SRC):
+        return "the reference's compiled CPU functions and its sources are not on this machine"
+    try:
+        oracle.build(ref=True)
+    except (OSError, subprocess.CalledProcessError) as e:
+        return f"the reference's CPU functions do not build here: {e!r}"[:300]
+    return None if os.path.exists(REF_LIB) else "building the reference's CPU functions left no library"
+
+
 def _ref_worker(q, path, N, L_slice, seed, core, warmup, steps):
     try:
         # the reference prints progress on stdout; keep the bench's stdout to one line
@@ -435,6 +452,8 @@ def run_ours(args):
     if world == 1 and not args.headline_only:
         ctx.close()
         out["other_configs"] = other_configs(not args.no_cpu_baseline)
+    if args.cpu_baseline_missing:
+        out["cpu_baseline"] = {"unavailable": args.cpu_baseline_missing}
     if cpu_rate is not None:
         out["cpu_baseline"] = {"value": round(cpu_rate, 5), "unit": METRIC, "cores": 1,
                                "kind": "reference", "sample": cpu_sample,
@@ -1012,11 +1031,22 @@ def main():
     args = ap.parse_args()
     if args.warmup < 3:
         args.warmup = 3
+    # without the reference's library the GPU's figures are printed all the same
+    args.cpu_baseline_missing = None
+    if args.impl == "reference" or not args.no_cpu_baseline:
+        args.cpu_baseline_missing = reference_missing()
+    if args.cpu_baseline_missing:
+        args.no_cpu_baseline = True
     if args.workload != "snp" and args.impl == "ours":
         {"grad": run_grad, "mala": run_mala, "scale": run_scale, "small": run_small,
          "uneven": run_uneven}[args.workload](args)
         return
     if args.impl == "reference":
+        if args.cpu_baseline_missing:
+            if int(os.environ.get("RANK", "0")) == 0:
+                print(json.dumps({"impl": "reference", "unavailable": args.cpu_baseline_missing}),
+                      flush=True)
+            return
         run_reference(args)
     else:
         run_ours(args)
