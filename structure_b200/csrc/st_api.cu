@@ -22,6 +22,8 @@ struct st_ctx {
   size_t budget = 0, in_use = 0;
   cudaStream_t stream = nullptr;       // launch stream (own or caller's)
   cudaStream_t own = nullptr;
+  bool lent = false;                   // has had a caller's stream
+  cudaEvent_t before_read = nullptr;   // the default stream's work at a st_get_state
   std::string err;
   int64_t launches = 0;
   bool profile = false;
@@ -444,6 +446,11 @@ extern "C" int st_ctx_create(int device, size_t hbm_budget, st_ctx** out) {
     delete ctx;
     return ST_ERR_CUDA;
   }
+  if (cudaEventCreateWithFlags(&ctx->before_read, cudaEventDisableTiming) != cudaSuccess) {
+    cudaStreamDestroy(ctx->own);
+    delete ctx;
+    return ST_ERR_CUDA;
+  }
   ctx->stream = ctx->own;
   *out = ctx;
   return ST_OK;
@@ -455,6 +462,7 @@ extern "C" int st_ctx_destroy(st_ctx* ctx) {
   cudaStreamSynchronize(ctx->stream);
   for (auto& e : ctx->evs) { cudaEventDestroy(e.a); cudaEventDestroy(e.b); }
   ctx_release_cache(ctx);
+  cudaEventDestroy(ctx->before_read);
   cudaStreamDestroy(ctx->own);
   delete ctx;
   return ST_OK;
@@ -463,6 +471,7 @@ extern "C" int st_ctx_destroy(st_ctx* ctx) {
 extern "C" int st_ctx_set_stream(st_ctx* ctx, void* stream) {
   if (!ctx) return ST_ERR_ARG;
   ctx->stream = stream ? (cudaStream_t)stream : ctx->own;
+  ctx->lent = ctx->lent || stream;
   return ST_OK;
 }
 
@@ -1531,8 +1540,16 @@ extern "C" int st_get_state(st_chain* c, int f, void* host, size_t bytes) {
   cudaStream_t s = c->ctx->stream;
   const ChainDev& h = c->h;
   // a copy behind the chain's work on its stream and one wait (a wait, then a copy on
-  // the default stream, took 17 us per field instead of 11)
+  // the default stream, took 17 us per field instead of 11).  Once the context has had
+  // a caller's stream, sweeps may also run on the default stream or on a blocking one
+  // that is not the context's now (a stream that it had before, a captured graph that
+  // is replayed there): the copy then follows those too, as one on the default stream
+  // does (half a microsecond more).
   auto read = [&](void* to, const void* from, size_t n) -> int {
+    if (c->ctx->lent && s != cudaStreamLegacy) {
+      ST_CUDA(c->ctx, cudaEventRecord(c->ctx->before_read, cudaStreamLegacy));
+      ST_CUDA(c->ctx, cudaStreamWaitEvent(s, c->ctx->before_read, 0));
+    }
     ST_CUDA(c->ctx, cudaMemcpyAsync(to, from, n, cudaMemcpyDeviceToHost, s));
     ST_CUDA(c->ctx, cudaStreamSynchronize(s));
     return ST_OK;
