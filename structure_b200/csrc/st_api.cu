@@ -703,6 +703,9 @@ extern "C" int st_data_upload(st_ctx* ctx, const st_data_desc* d, st_data** out)
     s->g2 = (uint32_t*)p;
     rc = cuda_check(ctx, cudaMemcpy(s->g2, src, sizeof(uint32_t) * (size_t)L * wpr,
                                     cudaMemcpyHostToDevice), "upload packed");
+    // (pageable copies on the default stream may still be under way, and the context's
+    // stream does not wait for them)
+    if (!rc) rc = cuda_check(ctx, cudaStreamSynchronize(cudaStreamLegacy), "upload packed");
     if (!rc && d->packed)
       rc = count_b2g_device(ctx, s->g2, N, L, wpr, A, s->cnt_h.data(), s->tot_h.data());
     if (rc) { st_data_destroy(s); return rc; }
@@ -1621,7 +1624,8 @@ extern "C" int st_set_state(st_chain* c, int f, const void* host, size_t bytes) 
   if (f == ST_F_DIMS || f == ST_F_LOGDIFF || f == ST_F_MYLOC)
     return seterr(c->ctx, ST_ERR_ARG, "field %d is read-only", f);
   if (f == ST_F_N || f == ST_F_M) {
-    // counts become partial slice 0; the other slices are cleared
+    // counts become partial slice 0; the other slices are cleared (behind the chain's
+    // queued sweeps, which write them)
     if (f == ST_F_N) {
       const size_t LKA = (size_t)h.L * h.K * h.A;
       std::vector<int32_t> part((size_t)h.cnt_chunks * LKA, 0);
@@ -1630,12 +1634,14 @@ extern "C" int st_set_state(st_chain* c, int f, const void* host, size_t bytes) 
         for (int a = 0; a < h.A; a++)
           for (int l = 0; l < h.L; l++)
             part[((size_t)k * h.A + a) * h.L + l] = in[((size_t)l * h.K + k) * h.A + a];
-      ST_CUDA(c->ctx, cudaMemcpy(h.npart, part.data(), part.size() * 4, cudaMemcpyHostToDevice));
+      ST_CUDA(c->ctx, cudaMemcpyAsync(h.npart, part.data(), part.size() * 4, cudaMemcpyHostToDevice, s));
+      ST_CUDA(c->ctx, cudaStreamSynchronize(s));
     } else {
       const size_t NK = (size_t)h.N * h.K;
       std::vector<int32_t> part((size_t)h.cnt_groups * NK, 0);
       memcpy(part.data(), host, NK * 4);
-      ST_CUDA(c->ctx, cudaMemcpy(h.mpart, part.data(), part.size() * 4, cudaMemcpyHostToDevice));
+      ST_CUDA(c->ctx, cudaMemcpyAsync(h.mpart, part.data(), part.size() * 4, cudaMemcpyHostToDevice, s));
+      ST_CUDA(c->ctx, cudaStreamSynchronize(s));
     }
     return ST_OK;
   }
@@ -1776,12 +1782,19 @@ static int batch_layout(st_batch* b, bool keep_groups) {
 
 static void batch_upload(st_batch* b) {
   const int n = (int)b->chains.size();
-  cudaMemcpy(b->d_table, b->table.data(), sizeof(ChainDev) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(b->d_pz, b->pz.data(), 4 * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(b->d_pzc, b->pzc.data(), 4 * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(b->d_pl, b->pl.data(), 4 * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(b->d_table_l, b->table_l.data(), sizeof(ChainDev) * n, cudaMemcpyHostToDevice);
-  cudaMemcpy(b->d_pi, b->pi.data(), 4 * n, cudaMemcpyHostToDevice);
+  // on the launches' stream: a copy on the default stream may still be under way when
+  // it returns, and the context's stream does not wait for it
+  cudaStream_t st = b->ctx->stream;
+  auto up = [&](void* to, const void* from, size_t bytes) {
+    cudaMemcpyAsync(to, from, bytes, cudaMemcpyHostToDevice, st);
+  };
+  up(b->d_table, b->table.data(), sizeof(ChainDev) * n);
+  up(b->d_pz, b->pz.data(), 4 * n);
+  up(b->d_pzc, b->pzc.data(), 4 * n);
+  up(b->d_pl, b->pl.data(), 4 * n);
+  up(b->d_table_l, b->table_l.data(), sizeof(ChainDev) * n);
+  up(b->d_pi, b->pi.data(), 4 * n);
+  cudaStreamSynchronize(st);
 }
 
 // Z-pass tile (T individuals per chunk, R locus blocks per CTA) of one chain;
@@ -2471,9 +2484,10 @@ extern "C" int st_chain_load(st_chain* c, const char* path) {
   if (!ok) return seterr(ctx, ST_ERR_STATE, "%s is truncated or of another chain", path);
   ST_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   for (size_t j = 0; j < fields.size(); j++)
-    if (cudaMemcpy(fields[j].p, bufs[j].data(), fields[j].bytes, cudaMemcpyHostToDevice) !=
-        cudaSuccess)
+    if (cudaMemcpyAsync(fields[j].p, bufs[j].data(), fields[j].bytes, cudaMemcpyHostToDevice,
+                        ctx->stream) != cudaSuccess)
       return seterr(ctx, ST_ERR_CUDA, "checkpoint upload failed");
+  ST_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
   c->h.key = key;
   c->h.cnt_chunks = 1;
   c->h.cnt_groups = 1;

@@ -92,3 +92,14 @@ def test_captured_sweeps_replayed_on_the_default_stream(words):
     del g
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("field", [api.F_N, api.F_M])
+def test_counts_set_behind_queued_sweeps(words, field):
+    a = Run(words, metrofreq=0)
+    want = np.ones((L, K, 2) if field == api.F_N else (N, K), np.int32)
+    a.chain.sweep(40)
+    a.chain.set(field, want)
+    assert a.chain.sync() == 0
+    np.testing.assert_array_equal(a.chain.get(field), want)
+    a.close()
