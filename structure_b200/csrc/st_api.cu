@@ -356,7 +356,7 @@ int zpass(st_chain* c, int mode, int flags) {
     return cuda_check(ctx, launch_u8(ls, c->KT, mode, flags, u8_smem(c->h, mode)), "zpass_u8");
   }
   if (c->model.precision == 1) flags |= kZfF64;
-  LaunchSet ls = single(c, ctas_zpass_u8(c->h, 256));
+  LaunchSet ls = single(c, ctas_zpass_u8(c->h));
   return cuda_check(ctx, launch_zpass_u8(ls, mode, flags), "zpass_u8");
 }
 
@@ -917,7 +917,7 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
   h.cnt_groups = 1;
 
   const size_t NK = (size_t)N * K, LKA = (size_t)L * K * A, LA = (size_t)L * A;
-  int zctas = c->fast ? ctas_zpass_b2g(h) : ctas_zpass_u8(h, 256);
+  int zctas = c->fast ? ctas_zpass_b2g(h) : ctas_zpass_u8(h);
   if (c->fast) {
     // room for the autotuner's smaller tiles (st_batch_autotune): T down to
     // half the chosen one at the chosen R
@@ -1739,7 +1739,7 @@ static int batch_layout(st_batch* b, bool keep_groups) {
       g.n++;
     } else {
       b->pz[j] = b->tz;
-      b->tz += ctas_zpass_u8(b->table[j], 256);
+      b->tz += ctas_zpass_u8(b->table[j]);
     }
     b->pi[j] = b->ti;
     b->ti += ctas_ind(b->table[j], kBlockInd);

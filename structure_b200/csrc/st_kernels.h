@@ -152,7 +152,7 @@ cudaError_t launch_init_chain(const ChainDev& h, ChainDev* d_chain, int* d_prefi
 
 // CTA counts per chain for each launch kind (host-side mirror of the tiling).
 int ctas_zpass_b2g(const ChainDev& c);
-int ctas_zpass_u8(const ChainDev& c, int block);
+int ctas_zpass_u8(const ChainDev& c);
 int ctas_locus(const ChainDev& c, int block);
 int locus_lanes(int L, int K, int A, long others);
 int ctas_ind(const ChainDev& c, int block);

@@ -197,8 +197,29 @@ cudaError_t launch_zmetro(const LaunchSet& ls, int KT, int flags, size_t smem) {
 // ---------------------------------------------------------------------------
 // Generic path: one thread per (individual, locus), any allele count, runtime
 // K, FP32 or FP64 arithmetic, Philox or injected uniforms.  Counts go to slice
-// 0 of the partial arrays with global atomics (zeroed by the host before).
+// 0 of the partial arrays with global atomics (zeroed by the host before), summed
+// over the CTA before that: thousands of copies share an individual's or, with many
+// individuals, a locus' few counts.
 // ---------------------------------------------------------------------------
+constexpr int kU8Threads = 256;
+constexpr int kU8Bins = 2048;   // allele counts of a CTA's loci kept in shared memory
+
+// Individuals of a CTA (a power of two up to 32, neighbouring lanes, as the genotypes
+// [L][N][2] lie) for at most an eighth of idle lanes; its loci are kU8Threads over that.
+__host__ __device__ inline int u8_inds(int N) {
+  int t = 32;
+  while (t > 1 && (N + t - 1) / t * t > N + N / 8) t >>= 1;
+  return t;
+}
+__host__ __device__ inline int u8_loci_tiles(int N, int L) {
+  const int loci = kU8Threads / u8_inds(N);
+  return (L + loci - 1) / loci;
+}
+__host__ __device__ inline int u8_tiles(int N, int L) {
+  const int inds = u8_inds(N);
+  return (N + inds - 1) / inds * u8_loci_tiles(N, L);
+}
+
 template <typename TF>
 __device__ __forceinline__ int pick_generic(const float* q, const float* Pl, int K, int A,
                                             int a, TF u, TF& total, int& errb);
@@ -242,15 +263,25 @@ __global__ void __launch_bounds__(256)
 zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains,
                 int mode, int flags) {
   __shared__ double sred[8];
+  __shared__ int sM[32 * kMaxPops], sN[kU8Bins];
   const int c = find_chain(prefix, nchains, blockIdx.x);
   ChainDev& ch = chains[c];
   const int tile = blockIdx.x - prefix[c];
   const int N = ch.N, L = ch.L, K = ch.K, A = ch.A;
-  // neighbouring threads are neighbouring individuals, as the genotypes [L][N][2] lie
-  const size_t idx = (size_t)tile * blockDim.x + threadIdx.x;
-  const bool active = idx < (size_t)N * L;
-  const int l = active ? (int)(idx / N) : 0;
-  const int i = active ? (int)(idx - (size_t)l * N) : 0;
+  const int inds = u8_inds(N), loci = kU8Threads / inds;
+  const int ltiles = u8_loci_tiles(N, L);
+  const int i0 = tile / ltiles * inds, l0 = tile % ltiles * loci;
+  const int ii = (int)threadIdx.x % inds, li = (int)threadIdx.x / inds;
+  const int i = i0 + ii, l = l0 + li;
+  const bool active = i < N && l < L;
+  const bool counts = mode == kZNormal || mode == kZInit || mode == kZRecount;
+  const bool binned = loci * K * A <= kU8Bins;
+  if (counts) {
+    for (int e = threadIdx.x; e < inds * K; e += kU8Threads) sM[e] = 0;
+    if (binned)
+      for (int e = threadIdx.x; e < loci * K * A; e += kU8Threads) sN[e] = 0;
+    __syncthreads();
+  }
   const int rep = *ch.rep;
   const bool collect = rep + 1 > ch.burnin;
   const bool want_like = (mode == kZLike) ||
@@ -308,15 +339,25 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
         if (mode != kZRecount && ch.Z && (flags & kZfStoreZ))
           ch.Z[((size_t)i * 2 + line) * L + l] = (uint8_t)z;
         if (mode == kZLike) continue;
-        atomicAdd(&ch.mpart[(size_t)i * K + z], 1);
-        if (!ch.pfrompopflagonly || ch.popflags[i] == 1)
-          atomicAdd(&ch.npart[((size_t)z * A + a) * L + l], 1);
+        atomicAdd(&sM[ii * K + z], 1);
+        if (!ch.pfrompopflagonly || ch.popflags[i] == 1) {
+          if (binned) atomicAdd(&sN[(z * A + a) * loci + li], 1);
+          else atomicAdd(&ch.npart[((size_t)z * A + a) * L + l], 1);
+        }
       }
     }
     if (mode == kZMetro) atomicAdd(&ch.ldpart[i], ld);
   }
   if (errb) set_err(ch.err, errb);
-  const int ntiles = (int)(((size_t)N * L + blockDim.x - 1) / blockDim.x);
+  if (counts) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < inds * K; e += kU8Threads)
+      if (sM[e]) atomicAdd(&ch.mpart[(size_t)i0 * K + e], sM[e]);
+    if (binned)
+      for (int e = threadIdx.x; e < loci * K * A; e += kU8Threads)
+        if (sN[e]) atomicAdd(&ch.npart[(size_t)(e / loci) * L + l0 + e % loci], sN[e]);
+  }
+  const int ntiles = u8_tiles(N, L);
   if (want_like) {
     double s = block_sum_d(like_acc, sred);
     if (threadIdx.x == 0) ch.likepart[tile] = s;
@@ -330,12 +371,10 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
   }
 }
 
-int ctas_zpass_u8(const ChainDev& c, int block) {
-  return (int)(((size_t)c.N * c.L + block - 1) / block);
-}
+int ctas_zpass_u8(const ChainDev& c) { return u8_tiles(c.N, c.L); }
 
 cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags) {
-  dim3 grid(ls.total_ctas), block(256);
+  dim3 grid(ls.total_ctas), block(kU8Threads);
   if (flags & kZfF64)
     zpass_u8_kernel<double><<<grid, block, 0, ls.stream>>>(ls.chains, ls.prefix, ls.nchains, mode, flags);
   else
