@@ -110,7 +110,8 @@ struct st_batch {
   int tz = 0, tl = 0, ti = 0;
   std::vector<ZGroup> zg;  // fast path: one Z launch per K class
   bool fast = false;
-  bool u8 = false;         // every chain takes st_zpass_u8.cu (one Z launch per K class)
+  bool u8 = false;         // chains take st_zpass_u8.cu: one Z launch per K class, and one
+                           // (class 0) for those that take the per-genotype kernel
   bool graphs = true;                          // replay captured sweeps
   cudaGraphExec_t gx[2] = {nullptr, nullptr};  // [Gibbs sweep, Metropolis sweep]
   int glaunches[2] = {0, 0};
@@ -912,6 +913,7 @@ extern "C" int st_chain_create(st_ctx* ctx, st_data* data, const st_model* model
     h.tileT = N; h.tileW = 8; h.tileR = 1;
     h.nchunks = 1;
     h.ngroups = 1;
+    set_zpass_u8_tile(&h);
   }
   h.cnt_chunks = 1;
   h.cnt_groups = 1;
@@ -1706,9 +1708,13 @@ static int batch_layout(st_batch* b, bool keep_groups) {
       }
       ZGroup& g = b->zg.back();   // (the autotuner, which keeps groups, has no tiles here)
       b->pz[j] = g.tz;
-      g.tz += ctas_u8(b->table[j]);
-      g.zsmem = std::max(g.zsmem, u8_smem(c->h, kZNormal));
-      g.msmem = std::max(g.msmem, u8_smem(c->h, kZMetro));
+      if (c->u8) {
+        g.tz += ctas_u8(b->table[j]);
+        g.zsmem = std::max(g.zsmem, u8_smem(c->h, kZNormal));
+        g.msmem = std::max(g.msmem, u8_smem(c->h, kZMetro));
+      } else {
+        g.tz += ctas_zpass_u8(b->table[j]);
+      }
       g.n++;
     } else if (b->fast) {
       if (!keep_groups && (b->zg.empty() || b->zg.back().KT != c->KT ||
@@ -1889,8 +1895,8 @@ extern "C" int st_batch_create(st_ctx* ctx, st_chain** chains, int n, st_batch**
                    });
   st_chain* c0 = b->chains[0];
   b->fast = c0->fast;
-  b->u8 = !c0->fast;
-  for (st_chain* c : b->chains) b->u8 = b->u8 && c->u8;
+  b->u8 = false;
+  for (st_chain* c : b->chains) b->u8 = b->u8 || c->u8;
   for (st_chain* c : b->chains) {
     if (c->ctx != ctx || c->fast != b->fast || c->h.metrofreq != c0->h.metrofreq ||
         c->host_rep != c0->host_rep || c->model.store_z != c0->model.store_z ||
@@ -2091,7 +2097,8 @@ static int enqueue_batch_sweep(st_batch* b, bool metro) {
       const int fl = flags | (g.same ? kZfInterleave : 0);
       if (b->u8) {
         LaunchSet lg{b->d_table + g.first, b->d_pz + g.first, g.n, g.tz, gs};
-        ST_CUDA(ctx, launch_u8(lg, g.KT, mode, flags, mode == kZMetro ? g.msmem : g.zsmem));
+        ST_CUDA(ctx, g.KT ? launch_u8(lg, g.KT, mode, flags, mode == kZMetro ? g.msmem : g.zsmem)
+                          : launch_zpass_u8(lg, mode, flags));
       } else if (g.count && mode == kZNormal) {
         LaunchSet lg{b->d_table + g.first, b->d_pzc + g.first, g.n, g.tzc, gs};
         ST_CUDA(ctx, launch_zcount(lg, g.KT, kZNormal, fl, g.zsmem_ct));

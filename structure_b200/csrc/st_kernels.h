@@ -114,7 +114,7 @@ size_t zmetro_smem(int KT, int T);
 cudaError_t launch_zmetro(const LaunchSet& ls, int KT, int flags, size_t smem);
 cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags);
 // One-byte layout, FP32 draws (st_zpass_u8.cu): modes kZNormal, kZLike and kZMetro.
-// u8_plan chooses the loci per chunk with at most `cap` CTAs; 0 if it cannot.
+// u8_plan chooses the loci per chunk with at most `cap` CTAs; 0: the per-genotype kernel.
 int u8_plan(int N, int L, int K, int A, long cap);
 int ctas_u8(const ChainDev& c);
 size_t u8_smem(const ChainDev& c, int mode);
@@ -152,6 +152,8 @@ cudaError_t launch_init_chain(const ChainDev& h, ChainDev* d_chain, int* d_prefi
 
 // CTA counts per chain for each launch kind (host-side mirror of the tiling).
 int ctas_zpass_b2g(const ChainDev& c);
+// CTAs of the per-genotype kernel, at the tile that set_zpass_u8_tile chose.
+void set_zpass_u8_tile(ChainDev* c);
 int ctas_zpass_u8(const ChainDev& c);
 int ctas_locus(const ChainDev& c, int block);
 int locus_lanes(int L, int K, int A, long others);

@@ -69,6 +69,7 @@ struct ChainDev {
   // Z-pass tiling: T individuals per chunk, W warps, R locus blocks per CTA
   int tileT, tileW, tileR, nchunks, ngroups;
   int u8_lc, u8_chunks;     // one-byte layout's Z pass: loci per chunk, chunks
+  int gen_shift, gen_ltiles;   // per-genotype kernel: log2 individuals per CTA, locus tiles
   // count histogram slices summed by the consumers (1: every producer adds
   // into slice 0); Metropolis log-ratio partials have ngroups slices
   int cnt_chunks, cnt_groups;

@@ -201,24 +201,8 @@ cudaError_t launch_zmetro(const LaunchSet& ls, int KT, int flags, size_t smem) {
 // over the CTA before that: thousands of copies share an individual's or, with many
 // individuals, a locus' few counts.
 // ---------------------------------------------------------------------------
-constexpr int kU8Threads = 256;
+constexpr int kU8Threads = 256;   // 2^8
 constexpr int kU8Bins = 2048;   // allele counts of a CTA's loci kept in shared memory
-
-// Individuals of a CTA (a power of two up to 32, neighbouring lanes, as the genotypes
-// [L][N][2] lie) for at most an eighth of idle lanes; its loci are kU8Threads over that.
-__host__ __device__ inline int u8_inds(int N) {
-  int t = 32;
-  while (t > 1 && (N + t - 1) / t * t > N + N / 8) t >>= 1;
-  return t;
-}
-__host__ __device__ inline int u8_loci_tiles(int N, int L) {
-  const int loci = kU8Threads / u8_inds(N);
-  return (L + loci - 1) / loci;
-}
-__host__ __device__ inline int u8_tiles(int N, int L) {
-  const int inds = u8_inds(N);
-  return (N + inds - 1) / inds * u8_loci_tiles(N, L);
-}
 
 template <typename TF>
 __device__ __forceinline__ int pick_generic(const float* q, const float* Pl, int K, int A,
@@ -268,10 +252,10 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
   ChainDev& ch = chains[c];
   const int tile = blockIdx.x - prefix[c];
   const int N = ch.N, L = ch.L, K = ch.K, A = ch.A;
-  const int inds = u8_inds(N), loci = kU8Threads / inds;
-  const int ltiles = u8_loci_tiles(N, L);
-  const int i0 = tile / ltiles * inds, l0 = tile % ltiles * loci;
-  const int ii = (int)threadIdx.x % inds, li = (int)threadIdx.x / inds;
+  const int inds = 1 << ch.gen_shift, loci = kU8Threads >> ch.gen_shift;
+  const int it = tile / ch.gen_ltiles;
+  const int i0 = it * inds, l0 = (tile - it * ch.gen_ltiles) * loci;
+  const int ii = (int)threadIdx.x & (inds - 1), li = (int)threadIdx.x >> ch.gen_shift;
   const int i = i0 + ii, l = l0 + li;
   const bool active = i < N && l < L;
   const bool counts = mode == kZNormal || mode == kZInit || mode == kZRecount;
@@ -355,9 +339,10 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
       if (sM[e]) atomicAdd(&ch.mpart[(size_t)i0 * K + e], sM[e]);
     if (binned)
       for (int e = threadIdx.x; e < loci * K * A; e += kU8Threads)
-        if (sN[e]) atomicAdd(&ch.npart[(size_t)(e / loci) * L + l0 + e % loci], sN[e]);
+        if (sN[e])
+          atomicAdd(&ch.npart[(size_t)(e >> (8 - ch.gen_shift)) * L + l0 + (e & (loci - 1))], sN[e]);
   }
-  const int ntiles = u8_tiles(N, L);
+  const int ntiles = (N + inds - 1) / inds * ch.gen_ltiles;
   if (want_like) {
     double s = block_sum_d(like_acc, sred);
     if (threadIdx.x == 0) ch.likepart[tile] = s;
@@ -371,7 +356,17 @@ zpass_u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, i
   }
 }
 
-int ctas_zpass_u8(const ChainDev& c) { return u8_tiles(c.N, c.L); }
+// Individuals of a CTA: a power of two up to 32, neighbouring lanes, as the genotypes
+// [L][N][2] lie, for at most an eighth of idle lanes; its loci are kU8Threads over that.
+void set_zpass_u8_tile(ChainDev* c) {
+  int s = 5;
+  while (s > 0 && (((c->N - 1) >> s) + 1) << s > c->N + c->N / 8) s--;
+  const int loci = kU8Threads >> s;
+  c->gen_shift = s;
+  c->gen_ltiles = (c->L - 1) / loci + 1;
+}
+
+int ctas_zpass_u8(const ChainDev& c) { return (((c.N - 1) >> c.gen_shift) + 1) * c.gen_ltiles; }
 
 cudaError_t launch_zpass_u8(const LaunchSet& ls, int mode, int flags) {
   dim3 grid(ls.total_ctas), block(kU8Threads);

@@ -155,7 +155,8 @@ u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nch
     const int spare = nl * K * A, KA = K * A;
     // the signs of the K - 1 thresholds: those of the class' padding count only where
     // a weight is negative (a caller may set any Q and P), and z then stays below K
-    const uint32_t zkeep = 0xFFFFFFFFu << (KT - K);
+    const uint32_t zkeep = KT == 3 || KT == 4 ? 0xFFFFFFFFu   // K = KT
+                                              : 0xFFFFFFFFu << (KT - K);
     int* myM = sM + threadIdx.x;
     LogProduct lp;
     // the pair's copies at a locus: two 16-bit loads side by side; individuals beyond
@@ -298,10 +299,17 @@ size_t u8_smem(const ChainDev& c, int mode) {
 // more copies: 8 chains of N=1000, L=300, K=6 take 37 us with 9 loci, 43 with 5; one
 // such chain 17.8 against 16.9), within the shared memory and the room for the
 // partials.  It depends on the chain's shape alone, so ln P(D) is the same in a batch.
+// 0: the per-genotype kernel, which also serves chains of few individuals: the P of a
+// chunk is then staged for few copies, more of them with more alleles and populations
+// (ten sweeps, us, per-genotype against tiled: 16 x 40,000, K=3, 2 alleles 921 / 1142,
+// 32 x 40,000 1411 / 1188; K=10, 6 alleles 16 x 5000 616 / 720, 48 x 5000 770 / 734;
+// K=20, 30 alleles 100 x 5000 3574 / 3968, 2 x 5000 2967 / 3880).  Chunks of one locus
+// fill the chip less than once either way, and stage less.
 int u8_plan(int N, int L, int K, int A, long cap) {
   const long blocks = (N + 2 * kUT - 1) / (2 * kUT);
   long lc = (L * blocks + 148 - 1) / 148;
   if (lc > kUMaxLc) lc = kUMaxLc;
+  if (lc > 1 && 4 * (long)(N - 18) < (long)K * A) return 0;
   const int KT = u8_kclass(K);
   while (lc > 1 && (u8_layout(KT, K, A, (int)lc, kZNormal).total > (int)kUSmem ||
                     u8_layout(KT, K, A, (int)lc, kZMetro).total > (int)kUSmem))
