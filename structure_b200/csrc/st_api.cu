@@ -354,6 +354,7 @@ int zpass(st_chain* c, int mode, int flags) {
     ST_CUDA(ctx, cudaMemsetAsync(c->h.ldpart, 0, sizeof(double) * (size_t)c->h.N, ctx->stream));
   if (c->u8 && u8_mode(mode) && !(flags & (kZfF64 | kZfInjected))) {
     LaunchSet ls = single(c, ctas_u8(c->h));
+    if (ctas_locus(c->h, kBlockLoc) <= 16) flags |= kZfEarly;
     return cuda_check(ctx, launch_u8(ls, c->KT, mode, flags, u8_smem(c->h, mode)), "zpass_u8");
   }
   if (c->model.precision == 1) flags |= kZfF64;

@@ -34,12 +34,17 @@ inline cudaError_t allow_dynamic_smem(F* fn, size_t smem) {
 // st_device.cuh's after_previous_kernel before it touches anything that a sweep's kernels
 // write.  What it reads before that (parameters, chain descriptors) must have been
 // written by a copy or by a kernel that an ordinary launch has followed since.
-// It lets the next kernel launch when its main loop is done, not at its start: blocks that
-// are there early only take up room (20,000 SNPs without admixture 303 us a sweep with
-// ordinary launches, 308 with the early signal, 295 with the late one).
-// A lone chain's sweeps ask for it: 200 individuals at 100 microsatellites go from 39 to
-// 30 us a sweep, 733 individuals at 9973 SNPs from 87 to 85, 1000 at 10,001 step by step
-// from 151 to 142.
+// The kernels do not signal before they end, so only the launch itself overlaps: blocks
+// that are there early take the SMs that are free first, up to four on one, and a locus
+// kernel of one to four blocks per SM then runs on some of the SMs while others idle.
+// Ten sweeps of a lone chain, us, ordinary launches / a signal behind each main loop /
+// none: 16 x 50,000 SNPs, K=10, F model 1524 / 1920 / 1447; 100 x 30,000, K=6 919 / 1017 /
+// 854; 733 x 9973, K=3 870 / 813 / 773; 2 x 3000, K=3 325 / 282 / 278; 2500 x 20,000, K=6
+// 2557 / 2485 / 2490.  Only the one-byte pass signals early (kZfEarly), where the locus
+// kernel behind it is of at most 16 blocks, too short for its place to matter (100
+// microsatellites of 20 individuals, K=3: 264 against 275; 20 of 200, K=2: 265 against
+// 280; but 1000 of 100, K=6, F model 602 against 503).
+// A lone chain's sweeps ask for it.
 template <typename... P, typename... A>
 inline cudaError_t launch_behind(const LaunchSet& ls, void (*fn)(P...), void (*fnb)(P...),
                                  unsigned block, size_t smem, A... args) {
@@ -72,6 +77,7 @@ enum : int {
   kZfF64 = 0x20,           // generic path: FP64 arithmetic (reference bit-parity)
   kZfInjected = 0x40,      // generic path: uniforms from the injected array
   kZfCleared = 0x100,      // the count histograms are zero already
+  kZfEarly = 0x200,        // the next kernel on the stream may launch before this one ends
   kZfInterleave = 0x80     // fast path: the launch's chains share one data set and
                            // tile, and block b runs tile b / nchains of chain
                            // b % nchains, so the chains' CTAs over the same loci run

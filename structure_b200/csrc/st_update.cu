@@ -324,7 +324,6 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
         ch.SumEps[(size_t)l * A + a] += ch.eps[(size_t)l * A + a];
   }
 
-  if (BEHIND) next_kernel_may_launch();
   // ---- F ------------------------------------------------------------------
   if (fstage) {
     // Each proposal's locus terms are summed as one balanced tree over the loci: within
@@ -672,7 +671,6 @@ ind_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nc
     }
   }
 
-  if (BEHIND) next_kernel_may_launch();
   if ((stages & kIndAlpha) && ch.inferalpha && mode != kIndPropose) {
     const int nslot = K + 1;
     const int nwarps = blockDim.x >> 5;

@@ -465,7 +465,6 @@ zcount_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int
     }
     __syncwarp();
   }
-  if (BEHIND) next_kernel_may_launch();
   __syncthreads();
   if constexpr (DRAW) {
     // thread = row: n_k = cum_{k-1} - cum_k, cum_{-1} = copies present

@@ -227,7 +227,7 @@ u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nch
       lp.flush();
       like_acc = lp.s;
     }
-    if (BEHIND) next_kernel_may_launch();
+    if (BEHIND && (flags & kZfEarly)) next_kernel_may_launch();
     if (MODE == kZNormal) {
       __syncthreads();
       for (int idx = threadIdx.x; idx < nl * K * A; idx += kUT) {   // locus fastest
