@@ -40,10 +40,13 @@ inline cudaError_t allow_dynamic_smem(F* fn, size_t smem) {
 // Ten sweeps of a lone chain, us, ordinary launches / a signal behind each main loop /
 // none: 16 x 50,000 SNPs, K=10, F model 1524 / 1920 / 1447; 100 x 30,000, K=6 919 / 1017 /
 // 854; 733 x 9973, K=3 870 / 813 / 773; 2 x 3000, K=3 325 / 282 / 278; 2500 x 20,000, K=6
-// 2557 / 2485 / 2490.  Only the one-byte pass signals early (kZfEarly), where the locus
+// 2557 / 2485 / 2490.  Two signal early: the one-byte pass (kZfEarly) where the locus
 // kernel behind it is of at most 16 blocks, too short for its place to matter (100
 // microsatellites of 20 individuals, K=3: 264 against 275; 20 of 200, K=2: 265 against
-// 280; but 1000 of 100, K=6, F model 602 against 503).
+// 280; but 1000 of 100, K=6, F model 602 against 503); and the locus kernel ahead of an F
+// stage or called by itself, with the short individual kernel behind it (1000 x 10,001,
+// K=4, an update at a time 77.0 against 78.8 us a step; 16 x 500, K=3 without F 284
+// against 271).
 // A lone chain's sweeps ask for it.
 template <typename... P, typename... A>
 inline cudaError_t launch_behind(const LaunchSet& ls, void (*fn)(P...), void (*fnb)(P...),

@@ -324,6 +324,9 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
         ch.SumEps[(size_t)l * A + a] += ch.eps[(size_t)l * A + a];
   }
 
+  // (launch_behind: early only before the F stage, whose last CTA the others wait for,
+  // or in an update called by itself)
+  if (BEHIND && (fstage || !(stages & (kLocClear | kLocCollect)))) next_kernel_may_launch();
   // ---- F ------------------------------------------------------------------
   if (fstage) {
     // Each proposal's locus terms are summed as one balanced tree over the loci: within
