@@ -16,6 +16,7 @@
 //                         PFROMPOPFLAGONLY
 //   one byte per copy     draws, ln P(D), Metropolis   st_zpass_u8.cu
 //                         the rest                     zpass_u8_kernel, below
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include "st_device.cuh"
@@ -128,9 +129,11 @@ CountTile zcount_tile(int N, int L, int KT, int tile_t, int tile_r, int chains, 
     return zcount_ctas(N, L, t) <= cap ? t : best;
   }
   double best_t = 1e300;
-  for (int n = 1; n <= (np + kZcountMinT - 1) / kZcountMinT; n++) {
+  // (each tile once: the count that gives the largest, then the next smaller one's)
+  for (int n = (N - 1) / kZcountMaxT + 1, next; n <= (np + kZcountMinT - 1) / kZcountMinT; n = next) {
     int T = ((N + n - 1) / n + 15) & ~15;
     if (T < kZcountMinT) T = kZcountMinT;
+    next = T > kZcountMinT ? std::max(n + 1, (N - 1) / (T - 16) + 1) : n + 1;
     if (!zcount_fits(KT, T)) continue;
     const CountTile c = with_r(T);
     const long ctas1 = zcount_ctas(N, L, c);
