@@ -222,10 +222,9 @@ __global__ void __launch_bounds__(kGradBlock) grad_loc_kernel(GradArgs a) {
 // ---------------------------------------------------------------------------
 // Two items (individuals or loci) per thread: 256 items per CTA.
 constexpr int k32Threads = kGradBlock / 2;
-#ifndef G32_CTAS
-#define G32_CTAS(KT) (KT <= 2 ? 6 : KT <= 4 ? 5 : KT <= 10 ? 4 : 3)
-#endif
-__host__ __device__ constexpr int g32_ctas(int KT) { return G32_CTAS(KT); }
+__host__ __device__ constexpr int g32_ctas(int KT) {
+  return KT <= 2 ? 6 : KT <= 4 ? 5 : KT <= 10 ? 4 : 3;
+}
 
 // S_0 S_1 and products of four genotype terms above this are far from FP32's range
 // ends, so their reciprocal and logarithm are as good as the factors' own; a group

@@ -33,7 +33,7 @@ constexpr int kNaPairs = 8;     // locus pairs per shared-memory stage (2-bit la
 template <int KC>
 __global__ void __launch_bounds__(kNaBlock)
 noadmix_ll_b2g_kernel(const ChainDev* __restrict__ chp) {
-  constexpr int kP = KC <= 16 ? kNaPairs : kNaPairs / 2;   // 32 KB of table at most
+  constexpr int kP = KC <= 16 ? kNaPairs : kNaPairs / 2;   // 16 KB of table at most
   __shared__ double2 tab[kP][KC / 2][16];   // class-minor: 8 classes span the banks
   __shared__ uint32_t sW[2 * kP][kNaBlock / 16];
   const ChainDev& ch = *chp;

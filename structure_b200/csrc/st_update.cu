@@ -1,6 +1,6 @@
 // st_update.cu -- the per-locus and per-individual updates of a sweep.
 //
-// Locus kernel (one thread per locus, a loop over the populations):
+// Locus kernel (a thread per locus, or up to 32 lanes where the loci are few):
 //   P   : P[l][k][.] ~ Dirichlet(prior + n[l][k][.])        Updates/UpdateP.c:106-199
 //   eps : two-allele shift Metropolis on eps[l][.]           Updates/UpdateEpsilon.c:71-145
 //   F   : per-locus terms of FlikeFreqs(F') - FlikeFreqs(F), reduced over loci,
@@ -83,9 +83,11 @@ __device__ __forceinline__ double warp_tree_sum(const double* p, size_t stride, 
 }  // namespace
 
 // ---------------------------------------------------------------------------
-// Locus kernel: one thread per locus, looping over the populations (every
-// lane busy whatever K is).  The per-population constants of the sweep --
-// (1-F_k)/F_k and the F proposals -- are formed once per CTA in shared memory.
+// Locus kernel: tpl lanes per locus, one where the loci fill the chip (a loop over the
+// populations then keeps every lane busy whatever K is).  With more, the lanes share
+// the populations and, in the P and F stages, the alleles; the eps move has one lane
+// per population.  The per-population constants of the sweep -- (1-F_k)/F_k and the F
+// proposals -- are formed once per CTA in shared memory.
 // ---------------------------------------------------------------------------
 constexpr int kStageKA = 16;   // populations x alleles staged per locus (P stage)
 
@@ -105,8 +107,7 @@ locus_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int 
   ChainDev& ch = chains[c];
   const int tile = blockIdx.x - prefix[c];
   const int L = ch.L, K = ch.K, A = ch.A;
-  // tpl lanes per locus (1 unless the chain has few loci): the P draws of a
-  // locus are spread over them; eps and F run on the first lane of each locus
+  // tpl lanes per locus (1 unless the chain has few loci)
   const int tpl = ch.loc_tpl;
   const int l = tile * ((int)blockDim.x / tpl) + (int)threadIdx.x / tpl;
   const int sub = (int)threadIdx.x % tpl;

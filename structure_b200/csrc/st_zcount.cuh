@@ -42,10 +42,10 @@ constexpr int kRedStride = 36;     // words per row of the reduction buffer (16-
 // 3 classes 102.5; 2 CTAs 113, 4 CTAs 108), K=8 143 (2 registers 147, two parts
 // 150, 2 CTAs 152), K=10 179 (4 registers 180, 3 CTAs 181, two parts 183,
 // shared-memory sums 186), K=20 382 (6 registers and 1 CTA 417, 14 registers
-// 391, four parts 392, shared-memory sums 528).  (K <= 5 has since lost 1.3 % more: the
-// likelihood product predicated, the loci's sign bytes added a pair of rows at a time.)  Where the table of every
-// population fits three CTAs, registers only add selects; above K=8 they make
-// room for two CTAs.
+// 391, four parts 392, shared-memory sums 528); taken before K <= 5 predicated its
+// likelihood product and added the loci's sign bytes a pair of rows at a time, which
+// made K=5 1.3 % faster.  Where the table of every population fits three CTAs, registers
+// only add selects; above K=8 they make room for two CTAs.
 __host__ __device__ constexpr int zc_ctas(int kt) { return kt <= 8 ? 3 : kt <= 24 ? 2 : 1; }
 __host__ __device__ constexpr int zc_nreg(int kt) {
   return kt <= 8 ? 0 : kt <= 12 ? 2 : kt <= 24 ? kt / 2 : 16;

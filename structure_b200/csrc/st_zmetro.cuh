@@ -24,9 +24,7 @@ constexpr float kTiny = 1e-30f;
 
 __host__ __device__ constexpr bool regp(int kt) { return kt <= 12; }
 __host__ __device__ constexpr int width(int kt) { return kt <= 12 ? 8 : 2; }   // warps
-#ifndef ZM_CTAS
-#define ZM_CTAS(kt) ((kt) <= 5 ? 3 : (kt) <= 12 ? 2 : 8)
-#endif
+__host__ __device__ constexpr int ctas(int kt) { return kt <= 5 ? 3 : kt <= 12 ? 2 : 8; }   // per SM
 
 struct Layout { int qt, x, ld, total; };
 
@@ -42,7 +40,7 @@ __host__ __device__ inline Layout layout(int kt, int T) {
 }
 
 template <int KT>
-__global__ void __launch_bounds__(32 * width(KT), ZM_CTAS(KT))
+__global__ void __launch_bounds__(32 * width(KT), ctas(KT))
 zmetro_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nchains, int flags) {
   extern __shared__ __align__(16) unsigned char smem[];
   constexpr int W = width(KT), NTH = 32 * W, KT2 = (KT + 1) & ~1;

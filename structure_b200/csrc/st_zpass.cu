@@ -7,9 +7,9 @@
 // The Metropolis Q move's likelihood ratio (CalcLike.c:281-345) and the initial random
 // Z (Init.c:125-169) are passes over the same data.
 //
-// This file holds the dispatchers, the tile rules, the generic path (FP64 arithmetic,
-// injected uniforms, stored Z on one-byte data) and the packing of one-byte data.  The
-// paths by data and chain:
+// This file holds the dispatchers, the tile rules, the per-genotype kernel of one-byte
+// data (FP64 arithmetic, injected uniforms, initial Z, counts of a given Z, chains of few
+// individuals) and the packing of that data.  The paths by data and chain:
 //   2 bits per genotype   draws and counts, ln P(D)    st_zcount.cuh
 //                         Metropolis ratio             st_zmetro.cuh
 //                         Init, recount; Z stored,     st_zpass_fast.cuh

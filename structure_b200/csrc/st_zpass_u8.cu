@@ -1,8 +1,9 @@
 // st_zpass_u8.cu -- the data pass on one-byte genotypes [L][N][2] (any allele count,
 // half-missing genotypes): the sweep's Z draws with counts and ln P(D), ln P(D) of a
-// state, and the Metropolis log ratios.  The initial Z, recounts, FP64 draws and
-// injected uniforms take the per-genotype kernel of st_zpass.cu; the draws here are
-// the same bits as that kernel's in FP32.
+// state, and the Metropolis log ratios; Z is stored where the chain keeps it.  The
+// initial Z, recounts, FP64 draws, injected uniforms and chains of few individuals
+// (u8_plan) take the per-genotype kernel of st_zpass.cu; the draws here are the same
+// bits as that kernel's in FP32.
 //
 // The layout puts individuals side by side, so that a warp reads the copies of 32 pairs
 // at a locus as one piece ([N][2][L] took a sector per byte: 56 instead of 37 us).
@@ -11,11 +12,12 @@
 // rows of an odd length: a copy reads its allele's row at fixed offsets, and lanes with
 // different alleles meet different banks.  Missing copies are counted as 0 or into a
 // spare slot, so that the loop has no branch but the rare logarithm (with branches and
-// rows [k][a] it took 647 warp instructions per 32 pairs and locus, 58 us).  Ancestry counts are lane-private columns in shared memory, allele
-// counts a histogram per CTA; both leave as one coalesced set of integer
-// reductions per CTA.  The per-genotype kernel added every copy to both
-// histograms with global atomics and took an FP64 logarithm per copy: 188 us per
-// sweep for 8 chains of N=1000, L=300, K=6, bound by those atomics' latency.
+// rows [k][a] it took 647 warp instructions per 32 pairs and locus, 58 us).  Ancestry
+// counts are lane-private columns in shared memory, allele counts a histogram per CTA;
+// both leave as one coalesced set of integer reductions per CTA.  A kernel that added
+// every copy to both histograms with global atomics and took an FP64 logarithm per copy
+// needed 188 us per sweep for 8 chains of N=1000, L=300, K=6, bound by those atomics'
+// latency.
 //
 // Logarithms: a thread multiplies its copies' terms in FP64 and takes one logarithm
 // whenever the product falls below 1e-100 (terms are at least 1e-50 after
