@@ -69,7 +69,6 @@ struct ChainDev {
   // Z-pass tiling: T individuals per chunk, W warps, R locus blocks per CTA
   int tileT, tileW, tileR, nchunks, ngroups;
   int u8_lc, u8_chunks;     // one-byte layout's Z pass: loci per chunk, chunks
-  int gen_shift, gen_ltiles;   // per-genotype kernel: log2 individuals per CTA, locus tiles
   // count histogram slices summed by the consumers (1: every producer adds
   // into slice 0); Metropolis log-ratio partials have ngroups slices
   int cnt_chunks, cnt_groups;
@@ -136,6 +135,8 @@ struct ChainDev {
   double *mLL, *mLLp;                   // [N] ll_i at current / proposed Q
   double *mTh, *mThp;                   // [N][K] logits (last fixed at 0)
   float* mEps;                          // [N] step sizes
+  // one-byte layout's per-genotype kernel: log2 individuals per CTA, locus tiles
+  int gen_shift, gen_ltiles;
 };
 
 }  // namespace st
