@@ -157,8 +157,8 @@ u8_kernel(ChainDev* __restrict__ chains, const int* __restrict__ prefix, int nch
     const int spare = nl * K * A, KA = K * A;
     // the signs of the K - 1 thresholds: those of the class' padding count only where
     // a weight is negative (a caller may set any Q and P), and z then stays below K
-    const uint32_t zkeep = KT == 3 || KT == 4 ? 0xFFFFFFFFu   // K = KT
-                                              : 0xFFFFFFFFu << (KT - K);
+    const uint32_t zkeep = KT <= 8 ? 0xFFFFFFFFu   // classes of one K
+                                   : 0xFFFFFFFFu << (KT - K);
     int* myM = sM + threadIdx.x;
     LogProduct lp;
     // the pair's copies at a locus: two 16-bit loads side by side; individuals beyond
@@ -285,7 +285,7 @@ cudaError_t launch_kt(const LaunchSet& ls, int mode, int flags, size_t smem) {
 }  // namespace
 
 int u8_kclass(int K) {
-  for (int k : {2, 3, 4, 6, 8, 12, 16, 24, 32})
+  for (int k : {1, 2, 3, 4, 5, 6, 7, 8, 10, 12, 16, 24, 32})
     if (k >= K) return k;
   return 0;
 }
@@ -327,8 +327,8 @@ int u8_plan(int N, int L, int K, int A, long cap) {
 cudaError_t launch_u8(const LaunchSet& ls, int KT, int mode, int flags, size_t smem) {
   switch (KT) {
 #define ST_KCASE(k) case k: return launch_kt<k>(ls, mode, flags, smem);
-    ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(6) ST_KCASE(8) ST_KCASE(12) ST_KCASE(16)
-    ST_KCASE(24) ST_KCASE(32)
+    ST_KCASE(1) ST_KCASE(2) ST_KCASE(3) ST_KCASE(4) ST_KCASE(5) ST_KCASE(6) ST_KCASE(7) ST_KCASE(8)
+    ST_KCASE(10) ST_KCASE(12) ST_KCASE(16) ST_KCASE(24) ST_KCASE(32)
 #undef ST_KCASE
   }
   return cudaErrorInvalidValue;
